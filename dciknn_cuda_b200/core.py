@@ -399,6 +399,11 @@ class DCI(object):
             raise RuntimeError(_capi.lib().dci_b200_last_error().decode())
         _capi.check(rc)
 
+    def set_pruning(self, mode):
+        """0 (default): leave out work that provably cannot change an answer where the sizes of the call make
+        it pay; 1: wherever possible; 2: never.  Results do not depend on it."""
+        _capi.check(_capi.lib().dci_b200_set_pruning(self._live(), int(mode)))
+
     def set_max_ctas(self, max_ctas):
         """Caps the number of CTAs of the traversal kernel (0 = automatic).  For tests: with few CTAs
         every CTA works through many (query, partition) pairs one after the other."""

@@ -6,6 +6,7 @@
 // (src/dci_cuda.cpp:54-173).
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdarg.h>
 #include <stdint.h>
 #include <stdio.h>
@@ -23,6 +24,8 @@
 #include "project.cuh"
 #include "project_tf32.cuh"
 #include "project_exact_tma.cuh"
+#include "distance_bounds.cuh"
+#include "prune.cuh"
 #include "traverse.cuh"
 
 namespace {
@@ -120,7 +123,8 @@ struct dci_b200 {
     int exact_tma = 1;                   // 0: never use the TMA-fed exact projection
     Buf keys, ids, pos, keysT;           // sorted index, inverse positions, stride-T keys: L*S*N entries each, partition-major (segment_start)
     int max_ctas = 0;                    // > 0: cap on the traversal grid (dci_b200_set_max_ctas)
-    Buf tmp_keys, qproj, part_topk, scratch, merge_scratch, stats, phases, hq, hids, hdists, qbound;
+    Buf tmp_keys, qproj, part_topk, scratch, merge_scratch, stats, phases, hq, hids, hdists, qbound, prune;
+    int pruning = 0;                     // 0: by the rule of prune_first_round, 1: wherever possible, 2: never
     int distance_bound = 1;              // 1: share a per-query distance bound between partitions
     int stats_on = 0, stats_nq = 0, phases_valid = 0;
     int timing_on = 0;
@@ -338,7 +342,7 @@ int launch_traverse(dci_b200 *h, dci::TraverseParams prm, int nthreads, cudaStre
     // ... and pays off when work items are exhaustive: lane 0 of a partition sees about ppb / T
     // promotions, so a quota well above that (with an iteration cap beyond the last window) is never met
     prm.qbatch = 1;
-    const bool likely_exhaustive = (long long)prm.max_cand * prm.T * 2 > 3ll * prm.ppb && prm.outer_s >= prm.wcap;
+    const bool likely_exhaustive = !prm.wl_offs && (long long)prm.max_cand * prm.T * 2 > 3ll * prm.ppb && prm.outer_s >= prm.wcap;
     if (smem && prm.vec8 && !prm.topk_global && !prm.blind && likely_exhaustive) {
         prm.dense_cap = next_pow2(prm.kpart + nthreads / 4);
         // per query a pair of selection buffers; for the group the query vectors, always kMaxQBatch slots
@@ -374,6 +378,111 @@ int launch_traverse(dci_b200 *h, dci::TraverseParams prm, int nthreads, cudaStre
     }
     h->launches++;
     DCI_CUDA(cudaGetLastError());
+    return 0;
+}
+
+// How a query call decides which (query, partition) pairs to traverse: 0 = all of them, otherwise the number of
+// partitions per query that round 1 visits (prune.cuh).
+// The bounds read every row once (6 TB/s) and multiply all queries with all rows (tf32, queries padded to tiles of
+// 128); a pair that need not be traversed saves about 0.31 ns of one SM per point and simple index (62 us for
+// 10 000 points x 20 indices), and k nearest rows spread evenly over P partitions leave
+// P * (1 - exp(-k / P)) of them to visit.  The factor 2 covers the small launches in between and the last
+// waves of the two rounds.
+int prune_first_round(const dci_b200 *h, const dci::TraverseParams &prm, int num_queries) {
+    if (prm.blind || prm.work_stats || prm.phase_cycles || !h->distance_bound || h->pruning == 2) return 0;
+    if (prm.num_parts < 2 || prm.ppb < 64) return 0;
+    const double parts = prm.num_parts, visited = 1.0 - exp(-1.1 * prm.knn / parts);
+    const double pairs = (double)num_queries * parts;
+    const double saved_us = (1.0 - visited) * pairs * 3.1e-4 * prm.ppb * prm.L * prm.S / h->sm_count;
+    const double padded = (double)((num_queries + dci::kLbQueries - 1) / dci::kLbQueries) * dci::kLbQueries;
+    const double cells = (double)prm.N * prm.dim;
+    const double cost_us = std::max(cells * 4.0 / 6.0e6, cells * padded * 2.0 / 0.35e9) + 40.0;
+    if (saved_us < 2.0 * cost_us && h->pruning != 1) return 0;
+    return std::min(prm.num_parts - 1, std::max(1, (int)(parts * visited + 0.5)));
+}
+
+// Working memory of a pruned batch, in 256-byte pieces: bounds | round-1 cut-offs | work lists | offsets |
+// [counters of both rounds | tickets | failure flag] (the bracketed part starts as zeros).
+struct PruneSpace {
+    size_t lb, thresh, list, offs, zero, bytes;
+    int zero_words;
+    static PruneSpace make(int parts, int nq) {
+        auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+        PruneSpace s;
+        s.lb = 0;
+        s.thresh = s.lb + up(sizeof(uint32_t) * (size_t)parts * nq);
+        s.list = s.thresh + up(sizeof(uint32_t) * (size_t)nq);
+        s.offs = s.list + up(sizeof(int) * (size_t)parts * nq);
+        s.zero = s.offs + up(sizeof(int) * ((size_t)parts + 1));
+        s.zero_words = 2 * parts + 3;
+        s.bytes = s.zero + up(sizeof(int) * (size_t)s.zero_words);
+        return s;
+    }
+};
+
+// Bounds of every (query, group of rows) of the batch prm.q0 .. prm.q0 + prm.nq.
+int launch_bounds(dci_b200 *h, const dci::TraverseParams &prm, int group_rows, int num_groups, uint32_t *lb, int *failed,
+                  cudaStream_t st) {
+    dci::BoundsParams bp;
+    memset(&bp, 0, sizeof(bp));
+    bp.data = prm.data; bp.query = prm.query + (size_t)prm.q0 * prm.dim;
+    bp.n = prm.N; bp.dim = prm.dim; bp.nq = prm.nq;
+    bp.group_rows = group_rows; bp.num_groups = num_groups; bp.q_stride = prm.nq;
+    bp.keep = (float)dci::bounds_keep(prm.dim);
+    bp.out = lb; bp.failed = failed;
+    // units of one tile of rows and as many query tiles as leave about four units per SM
+    const int row_tiles = (prm.N + dci::kLbRows - 1) / dci::kLbRows, q_tiles = (prm.nq + dci::kLbQueries - 1) / dci::kLbQueries;
+    const int want = std::max(1, std::min(q_tiles, (4 * h->sm_count + row_tiles - 1) / row_tiles));
+    bp.qt_per_unit = (q_tiles + want - 1) / want;
+    bp.units_q = (q_tiles + bp.qt_per_unit - 1) / bp.qt_per_unit;
+    const unsigned grid = (unsigned)std::min<long long>((long long)row_tiles * bp.units_q, h->sm_count);
+    CUtensorMap map_x, map_q;
+    memset(&map_x, 0, sizeof(map_x));
+    memset(&map_q, 0, sizeof(map_q));
+    const bool tma = make_tensor_map_2d(&map_x, bp.data, bp.n, bp.dim, dci::kLbRows) &&
+                     make_tensor_map_2d(&map_q, bp.query, bp.nq, bp.dim, dci::kLbQueries);
+    auto go = [&](auto kern) -> int {
+        DCI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dci::kLbSmem));
+        kern<<<grid, dci::kLbThreads, dci::kLbSmem, st>>>(map_x, map_q, bp);
+        h->launches++;
+        DCI_CUDA(cudaGetLastError());
+        return 0;
+    };
+    return tma ? go(dci::distance_bounds_kernel<false>) : go(dci::distance_bounds_kernel<true>);
+}
+
+// One batch with pruning: bounds, then the two rounds.  traverse(prm) launches the traversal of prm's work list.
+// ws: PruneSpace::make(num_parts, nq).bytes of device memory; prm.qbound and prm.part_topk are set.
+template <typename Traverse>
+int traverse_pruned(dci_b200 *h, dci::TraverseParams prm, int first, unsigned char *ws, cudaStream_t st, Traverse traverse) {
+    const PruneSpace sp = PruneSpace::make(prm.num_parts, prm.nq);
+    uint32_t *lb = (uint32_t *)(ws + sp.lb);
+    int *zero = (int *)(ws + sp.zero);
+    const size_t topk_words = (size_t)prm.nq * prm.num_parts * prm.kpart;      // 8 bytes each, 16-byte aligned array
+    dci::prune_init_kernel<<<h->sm_count * 4, 256, 0, st>>>((uint4 *)prm.part_topk, (topk_words + 1) / 2, lb,
+                                                            (size_t)prm.num_parts * prm.nq, prm.qbound, prm.nq, zero, sp.zero_words);
+    h->launches++;
+    DCI_CUDA(cudaGetLastError());
+    dci::SelectParams s;
+    memset(&s, 0, sizeof(s));
+    int *failed = zero + 2 * prm.num_parts + 2;
+    if (int rc = launch_bounds(h, prm, prm.ppb, prm.num_parts, lb, failed, st)) return rc;
+    s.lb = lb; s.failed = failed;
+    s.query = prm.query + (size_t)prm.q0 * prm.dim;
+    s.part_topk = prm.part_topk; s.thresh = (uint32_t *)(ws + sp.thresh); s.qbound = prm.qbound;
+    s.offs = (int *)(ws + sp.offs); s.list = (int *)(ws + sp.list);
+    s.nq = prm.nq; s.num_groups = prm.num_parts; s.q_stride = prm.nq; s.first = first; s.knn = prm.knn; s.kpart = prm.kpart;
+    s.dim = prm.dim; s.keep = (float)dci::bounds_keep(prm.dim);
+    prm.wl_offs = s.offs; prm.wl_list = s.list; prm.wl_stride = prm.nq;
+    for (int round = 1; round <= 2; ++round) {
+        s.cnt = zero + (round - 1) * prm.num_parts;
+        s.ticket = zero + 2 * prm.num_parts + (round - 1);
+        if (round == 1) dci::select_work_kernel<1><<<prm.nq, 128, 0, st>>>(s);
+        else dci::select_work_kernel<2><<<prm.nq, 128, 0, st>>>(s);
+        h->launches++;
+        DCI_CUDA(cudaGetLastError());
+        if (int rc = traverse(prm)) return rc;
+    }
     return 0;
 }
 
@@ -434,7 +543,7 @@ int dci_b200_destroy(dci_b200_t *h) {
     if (!h) return 0;
     DeviceGuard g(h->device);
     cudaDeviceSynchronize();
-    Buf *bufs[] = {&h->keys, &h->ids, &h->pos, &h->keysT, &h->tmp_keys, &h->qproj, &h->part_topk, &h->scratch, &h->merge_scratch, &h->stats, &h->phases, &h->errflag, &h->qbound,
+    Buf *bufs[] = {&h->keys, &h->ids, &h->pos, &h->keysT, &h->tmp_keys, &h->qproj, &h->part_topk, &h->scratch, &h->merge_scratch, &h->stats, &h->phases, &h->errflag, &h->qbound, &h->prune,
                    &h->hq, &h->hids, &h->hdists};
     for (Buf *b : bufs) b->release();
     if (h->d_proj) counted_free(h->d_proj);
@@ -650,7 +759,6 @@ static int query_impl(dci_b200_t *h, const float *d_query, int num_queries, int 
     DeviceGuard g(h->device);
     cudaStream_t st = (cudaStream_t)stream;
     const int I = h->L * h->S;
-    DCI_CUDA(h->qproj.ensure(sizeof(float) * (size_t)I * num_queries));
     const bool timing = h->timing_on != 0;
     if (timing) {
         for (auto &e : h->ev) if (!e) DCI_CUDA(cudaEventCreate(&e));
@@ -658,14 +766,12 @@ static int query_impl(dci_b200_t *h, const float *d_query, int num_queries, int 
         h->t_traverse_launches = 0;
         DCI_CUDA(cudaEventRecord(h->ev[0], st));
     }
-    if (int rc = launch_project(h, d_query, num_queries, (float *)h->qproj.p, st)) return rc;
-    if (timing) DCI_CUDA(cudaEventRecord(h->ev[1], st));
 
     dci::TraverseParams prm;
     memset(&prm, 0, sizeof(prm));
     prm.skeys = (const float *)h->keys.p; prm.skeysT = (const float *)h->keysT.p; prm.sids = (const int *)h->ids.p;
     prm.spos = h->pos.p; prm.data = h->d_data;
-    prm.qproj = (const float *)h->qproj.p; prm.query = d_query;
+    prm.query = d_query;
     prm.N = h->num_points; prm.dim = h->dim; prm.L = h->L; prm.S = h->S; prm.P = h->P; prm.T = h->T;
     prm.ppb = h->ppb; prm.num_parts = h->num_parts; prm.nq_total = num_queries;
     prm.knn = num_neighbours; prm.max_cand = max_num_candidates;
@@ -700,9 +806,15 @@ static int query_impl(dci_b200_t *h, const float *d_query, int num_queries, int 
         prm.work_stats = (long long *)h->stats.p;
         h->stats_nq = num_queries;
     }
+    DCI_CUDA(h->qproj.ensure(sizeof(float) * (size_t)I * num_queries));
+    prm.qproj = (const float *)h->qproj.p;
+    if (int rc = launch_project(h, d_query, num_queries, (float *)h->qproj.p, st)) return rc;
+    if (timing) DCI_CUDA(cudaEventRecord(h->ev[1], st));
     const size_t per_query = sizeof(uint64_t) * (size_t)h->num_parts * prm.kpart;
     const int batch = (int)std::max<size_t>(1, std::min<size_t>((size_t)num_queries, ((size_t)1 << 30) / per_query));
-    DCI_CUDA(h->part_topk.ensure(per_query * batch));
+    DCI_CUDA(h->part_topk.ensure(per_query * batch + 16));
+    const int prune_first = prune_first_round(h, prm, std::min(batch, num_queries));
+    if (prune_first) DCI_CUDA(h->prune.ensure(PruneSpace::make(h->num_parts, batch).bytes));
     prm.part_topk = (uint64_t *)h->part_topk.p;
     const int merge_grid_cap = merge_global ? 2 * h->sm_count : (1 << 30);
     if (merge_global) DCI_CUDA(h->merge_scratch.ensure((size_t)merge_grid_cap * 2 * merge_cap * sizeof(uint64_t)));
@@ -712,7 +824,8 @@ static int query_impl(dci_b200_t *h, const float *d_query, int num_queries, int 
         prm.nq = std::min(batch, num_queries - q0);
         if (h->distance_bound && !blind) {
             prm.qbound = (uint32_t *)h->qbound.p;
-            DCI_CUDA(cudaMemsetAsync(prm.qbound, 0x7F, sizeof(uint32_t) * (size_t)prm.nq, st));   // 0x7F7F7F7F: a huge finite float
+            if (!prune_first)
+                DCI_CUDA(cudaMemsetAsync(prm.qbound, 0x7F, sizeof(uint32_t) * (size_t)prm.nq, st));   // 0x7F7F7F7F: a huge finite float
         }
         if (timing) DCI_CUDA(cudaEventRecord(h->ev[2], st));
         int rc;
@@ -731,11 +844,14 @@ static int query_impl(dci_b200_t *h, const float *d_query, int num_queries, int 
             h->last_qbatch = 1;
             DCI_CUDA(cudaGetLastError());
             rc = 0;
-        } else if (pos16(prm.ppb, h->T))
-            rc = (prm.wcap <= 65535) ? launch_traverse<uint16_t, uint16_t>(h, prm, nthreads, st)
-                                     : launch_traverse<uint32_t, uint16_t>(h, prm, nthreads, st);
-        else
-            rc = launch_traverse<uint32_t, uint32_t>(h, prm, nthreads, st);
+        } else {
+            auto traverse = [&](const dci::TraverseParams &p) -> int {
+                if (!pos16(p.ppb, h->T)) return launch_traverse<uint32_t, uint32_t>(h, p, nthreads, st);
+                return p.wcap <= 65535 ? launch_traverse<uint16_t, uint16_t>(h, p, nthreads, st)
+                                       : launch_traverse<uint32_t, uint16_t>(h, p, nthreads, st);
+            };
+            rc = prune_first ? traverse_pruned(h, prm, prune_first, (unsigned char *)h->prune.p, st, traverse) : traverse(prm);
+        }
         if (rc) return rc;
         if (timing) DCI_CUDA(cudaEventRecord(h->ev[3], st));
         dci::merge_partitions_kernel<<<std::min(prm.nq, merge_grid_cap), merge_threads,
@@ -907,6 +1023,13 @@ int dci_b200_set_max_ctas(dci_b200_t *h, int max_ctas) {
     if (int rc = check_handle(h)) return rc;
     if (max_ctas < 0) return fail(DCI_B200_ERR_ARG, "max_ctas must not be negative");
     h->max_ctas = max_ctas;
+    return 0;
+}
+
+int dci_b200_set_pruning(dci_b200_t *h, int mode) {
+    if (int rc = check_handle(h)) return rc;
+    if (mode < 0 || mode > 2) return fail(DCI_B200_ERR_ARG, "pruning mode must be 0 (automatic), 1 (always) or 2 (never)");
+    h->pruning = mode;
     return 0;
 }
 
@@ -1261,7 +1384,7 @@ size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 template <typename ValT, typename PosT>
 int query_noalloc_impl(dci_b200 *h, dci::TraverseParams prm, int nthreads, unsigned char *scratch, size_t avail,
-                       int num_queries, int *d_ids, float *d_dists, cudaStream_t st) {
+                       int num_queries, int *flag_word, int *d_ids, float *d_dists, cudaStream_t st) {
     cudaFuncAttributes fa;
     DCI_CUDA(cudaFuncGetAttributes(&fa, dci::traverse_kernel<ValT, PosT, true, true>));
     const size_t static_smem = fa.sharedSizeBytes;
@@ -1279,11 +1402,18 @@ int query_noalloc_impl(dci_b200 *h, dci::TraverseParams prm, int nthreads, unsig
     const size_t slabs = per_cta * (size_t)max_grid;
     // per query of a pass: its per-partition result lists and its word of the shared distance bound
     const size_t per_query = sizeof(uint64_t) * (size_t)prm.num_parts * prm.kpart + sizeof(uint32_t);
+    int prune_first = prune_first_round(h, prm, num_queries);
     if (slabs + per_query + 256 > avail)
         return fail(DCI_B200_ERR_UNSUPPORTED,
                     "this index and k need %zu bytes of working memory, the built-in scratch of the allocation-free query holds %u",
                     slabs + per_query + 256 + ((size_t)DCI_B200_NOALLOC_SCRATCH_BYTES - avail), (unsigned)DCI_B200_NOALLOC_SCRATCH_BYTES);
+    // the handle's own flag word and timing events are created on first use, so neither is used here
+    if (int rc = launch_project(h, prm.query, num_queries, const_cast<float *>(prm.qproj), st, flag_word, false)) return rc;
     const int batch = (int)std::min<size_t>((size_t)num_queries, (avail - slabs - 256) / per_query);
+    // pruning (as in the regular query) where one pass over all queries and its lists fit beside the rest
+    const size_t lists_end = slabs + align256(sizeof(uint64_t) * (size_t)prm.num_parts * prm.kpart * batch) +
+                             align256(sizeof(uint32_t) * (size_t)batch);
+    if (batch < num_queries || lists_end + PruneSpace::make(prm.num_parts, batch).bytes > avail) prune_first = 0;
     prm.gscratch = scratch;
     prm.gscratch_per_cta = per_cta;
     prm.part_topk = (uint64_t *)(scratch + slabs);
@@ -1303,12 +1433,16 @@ int query_noalloc_impl(dci_b200 *h, dci::TraverseParams prm, int nthreads, unsig
         prm.nq = std::min(batch, num_queries - q0);
         if (qbound) {      // the bound words must start as "no bound yet": the array keeps the last call's contents
             prm.qbound = qbound;
-            DCI_CUDA(cudaMemsetAsync(qbound, 0x7F, sizeof(uint32_t) * (size_t)prm.nq, st));
+            if (!prune_first) DCI_CUDA(cudaMemsetAsync(qbound, 0x7F, sizeof(uint32_t) * (size_t)prm.nq, st));
         }
         const unsigned grid = (unsigned)std::min<long long>((long long)prm.nq * prm.num_parts, max_grid);
-        kern<<<grid, nthreads, dyn, st>>>(prm);
-        h->launches++;
-        DCI_CUDA(cudaGetLastError());
+        auto traverse = [&](const dci::TraverseParams &p) -> int {
+            kern<<<grid, nthreads, dyn, st>>>(p);
+            h->launches++;
+            DCI_CUDA(cudaGetLastError());
+            return 0;
+        };
+        if (int rc = prune_first ? traverse_pruned(h, prm, prune_first, scratch + lists_end, st, traverse) : traverse(prm)) return rc;
         dci::merge_partitions_kernel<<<prm.nq, merge_threads, (size_t)merge_cap * 16, st>>>(
             prm.part_topk, prm.num_parts, prm.kpart, prm.knn, merge_cap, q0, prm.nq, nullptr, d_ids, d_dists, 0);
         h->launches++;
@@ -1347,9 +1481,6 @@ extern "C" int dci_b200_query_noalloc(dci_b200_t *h, const float *d_query, int n
         return fail(DCI_B200_ERR_UNSUPPORTED, "%d queries need %zu bytes for their projections alone, the built-in scratch holds %u",
                     num_queries, qproj_bytes, (unsigned)DCI_B200_NOALLOC_SCRATCH_BYTES);
     float *qproj = (float *)(scratch + 256);
-    // the handle's own flag word and timing events are created on first use, so neither is used here
-    if (int rc = launch_project(h, d_query, num_queries, qproj, st, (int *)scratch, false)) return rc;
-
     dci::TraverseParams prm;
     memset(&prm, 0, sizeof(prm));
     prm.skeys = (const float *)h->keys.p; prm.skeysT = (const float *)h->keysT.p; prm.sids = (const int *)h->ids.p;
@@ -1372,7 +1503,7 @@ extern "C" int dci_b200_query_noalloc(dci_b200_t *h, const float *d_query, int n
     const size_t avail = (size_t)DCI_B200_NOALLOC_SCRATCH_BYTES - 256 - qproj_bytes;
     if (pos16(prm.ppb, h->T))
         return (prm.wcap <= 65535)
-                   ? query_noalloc_impl<uint16_t, uint16_t>(h, prm, nthreads, rest, avail, num_queries, d_ids, d_dists, st)
-                   : query_noalloc_impl<uint32_t, uint16_t>(h, prm, nthreads, rest, avail, num_queries, d_ids, d_dists, st);
-    return query_noalloc_impl<uint32_t, uint32_t>(h, prm, nthreads, rest, avail, num_queries, d_ids, d_dists, st);
+                   ? query_noalloc_impl<uint16_t, uint16_t>(h, prm, nthreads, rest, avail, num_queries, (int *)scratch, d_ids, d_dists, st)
+                   : query_noalloc_impl<uint32_t, uint16_t>(h, prm, nthreads, rest, avail, num_queries, (int *)scratch, d_ids, d_dists, st);
+    return query_noalloc_impl<uint32_t, uint32_t>(h, prm, nthreads, rest, avail, num_queries, (int *)scratch, d_ids, d_dists, st);
 }

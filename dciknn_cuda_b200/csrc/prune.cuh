@@ -1,0 +1,129 @@
+// Which (query, partition) pairs have to be traversed.
+//
+// Only a query's k nearest candidates over all partitions reach its result, so a partition whose nearest row
+// lies strictly beyond k candidates that are already known cannot change the answer.  distance_bounds_kernel
+// gives a rigorous lower bound of the nearest row of every partition; the pairs are then traversed in two
+// rounds.  Round 1: per query the partitions with the smallest bounds, about as many as hold the k nearest
+// rows when rows are spread evenly.  Round 2: every other partition whose bound does not exceed the k-th best
+// candidate of round 1 -- all of them when round 1 found fewer than k.  A pair that is left out keeps an empty
+// list.  Nothing is assumed about the data: clustered rows only make the lists shorter, and a distribution on
+// which the index finds few near neighbours (a loose k-th candidate) makes round 2 traverse more.
+#pragma once
+#include "common.cuh"
+
+namespace dci {
+
+struct SelectParams {
+    const uint32_t *lb;           // [num_groups][q_stride], see distance_bounds.cuh
+    const int *failed;            // not 0: the bounds are unusable, every pair is traversed in round 1
+    const float *query;           // rows q0 .. of the call's queries
+    uint64_t *part_topk;          // [nq][num_groups][kpart], empty lists where nothing was traversed
+    uint32_t *thresh;             // [nq] round 1's cut-off
+    uint32_t *qbound;             // [nq] the shared distance bound of the traversal
+    int *cnt, *offs, *list;       // [num_groups] (starts as 0), [num_groups + 1], [num_groups][q_stride]
+    int *ticket;                  // starts as 0
+    int nq, num_groups, q_stride, first, knn, kpart, dim;
+    float keep;
+};
+
+// Starting values of everything the rounds use, in one launch: empty lists, no bound yet, bounds and counters.
+__global__ void prune_init_kernel(uint4 *topk, size_t topk16, uint32_t *lb, size_t lb_words, uint32_t *qbound, int nq,
+                                  int *zero, int zero_words) {
+    const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = i0; i < topk16; i += step) topk[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    for (size_t i = i0; i < lb_words; i += step) lb[i] = ~0u;
+    for (size_t i = i0; i < (size_t)nq; i += step) qbound[i] = 0x7F7F7F7Fu;      // no bound yet
+    for (size_t i = i0; i < (size_t)zero_words; i += step) zero[i] = 0;
+}
+
+// One CTA per query.  Appends the query to the work lists of the partitions it has to visit in this round; the
+// last CTA to finish turns the list lengths into offsets.
+template <int ROUND>
+__global__ void __launch_bounds__(128) select_work_kernel(const SelectParams p) {
+    __shared__ uint32_t s_sel[2][256];
+    __shared__ uint32_t s_res[4];
+    __shared__ double s_sum[4];
+    __shared__ int s_last;
+    __shared__ uint32_t s_scratch[40];
+    const int q = blockIdx.x, tid = threadIdx.x;
+    const uint32_t *lb = p.lb + q;
+    const size_t stride = (size_t)p.q_stride;
+    uint32_t lo = 0u;                 // bounds above lo (ROUND 2) ...
+    float limit = __int_as_float(0x7F800000);      // ... and not beyond limit are taken
+    uint32_t hi = 0xFFFFFFFFu;        // ROUND 1: bounds up to hi are taken
+    if (ROUND == 1) {
+        if (!*p.failed && p.first < p.num_groups) {
+            uint32_t out[2];
+            cta_select2([lb, stride](int j) { return lb[(size_t)j * stride]; }, p.num_groups, p.first, p.first, 32, s_sel, s_res, out);
+            hi = out[0];
+        }
+        if (tid == 0) p.thresh[q] = hi;
+    } else {
+        lo = p.thresh[q];
+        if (lo != 0xFFFFFFFFu) {      // the same for every thread
+            // k-th best candidate of round 1
+            const uint64_t *lists = p.part_topk + (size_t)q * p.num_groups * p.kpart;
+            const int total = p.num_groups * p.kpart;
+            uint32_t kth = 0xFFFFFFFFu;
+            if (p.knn <= total) {
+                uint32_t out[2];
+                cta_select2([lists](int j) { return (uint32_t)(lists[j] >> 32); }, total, p.knn, p.knn, 32, s_sel, s_res, out);
+                kth = out[0];
+            }
+            double s = 0.0;           // |q|^2
+            for (int c = tid; c < p.dim; c += blockDim.x) { const double v = p.query[(size_t)q * p.dim + c]; s += v * v; }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
+            if ((tid & 31) == 0) s_sum[tid >> 5] = s;
+            __syncthreads();
+            const double q2 = (s_sum[0] + s_sum[1]) + (s_sum[2] + s_sum[3]);
+            const float d = __uint_as_float(kth);              // an empty slot reads as NaN
+            if (d < __int_as_float(0x7F800000) && q2 <= 1.0e30) {
+                // a row is strictly beyond d when its squared distance exceeds d^2 by more than the rounding of
+                // the distance chain (about (dim + 4) 2^-24, twice that taken); 1e-18 covers underflow
+                const double t = (double)d * d * (1.0 + (p.dim + 8.0) / 8388608.0) + 1.0e-18 - (double)p.keep * q2;
+                limit = __double2float_ru(t);
+                if (tid == 0) atomicMin(p.qbound + q, kth);
+            }
+        }
+    }
+    if (ROUND == 1 || lo != 0xFFFFFFFFu) {
+        for (int g = tid; g < p.num_groups; g += blockDim.x) {
+            const uint32_t v = lb[(size_t)g * stride];
+            const bool take = ROUND == 1 ? v <= hi : (v > lo && !(ordered_to_float(v) > limit));
+            if (take) p.list[(size_t)g * stride + atomicAdd(p.cnt + g, 1)] = q;
+        }
+    }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(p.ticket, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (s_last) {
+        __threadfence();
+        // exclusive scan of the list lengths, blockDim.x of them at a time
+        int run = 0;
+        for (int g0 = 0; g0 < p.num_groups; g0 += blockDim.x) {
+            const int g = g0 + tid, lane = tid & 31;
+            const int c = g < p.num_groups ? __ldcg(p.cnt + g) : 0;
+            int inc = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+                if (lane >= o) inc += t;
+            }
+            if (lane == 31) s_scratch[tid >> 5] = (uint32_t)inc;
+            __syncthreads();
+            int before = run, total = 0;
+            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
+                if (w < (tid >> 5)) before += (int)s_scratch[w];
+                total += (int)s_scratch[w];
+            }
+            if (g < p.num_groups) p.offs[g] = before + inc - c;
+            run += total;
+            __syncthreads();
+        }
+        if (tid == 0) p.offs[p.num_groups] = run;
+    }
+}
+
+}  // namespace dci

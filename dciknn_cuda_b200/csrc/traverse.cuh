@@ -71,6 +71,9 @@ struct TraverseParams {
     int dense_cap;             // capacity of the dense pass's selection buffers: power of two >= kpart + blockDim/4
     uint32_t *qbound;          // nullptr or [nq]: per query of this launch, fp32 bits of an upper bound of its k-th
                                // smallest distance found so far (any partition); candidates beyond it are dropped
+    const int *wl_offs;        // nullptr (every pair), or the pairs to traverse: offsets [num_parts + 1] into ...
+    const int *wl_list;        // ... the queries of each partition, [num_parts][wl_stride] (prune.cuh)
+    int wl_stride;
     int blind;                 // 1: no distances; a promoted point's key is its promotion iteration (needs topk_global)
     FastDiv divT;
 };
@@ -391,7 +394,8 @@ traverse_kernel(const TraverseParams prm) {
     // deferred and their distances computed in one pass that loads each row once for all of them.
     const int Q = BATCH ? (prm.qbatch > 0 ? prm.qbatch : 1) : 1;
     const int ngroups = (prm.nq + Q - 1) / Q;
-    const long long nwork = (long long)ngroups * prm.num_parts;
+    const bool listed = !BATCH && prm.wl_offs != nullptr;
+    const long long nwork = listed ? (long long)prm.wl_offs[prm.num_parts] : (long long)ngroups * prm.num_parts;
     long long t_last = 0;
 #define DCI_PHASE_MARK(slot_)                                                             \
     if (f_phase_cycles && tid == 0) {                                                   \
@@ -401,7 +405,16 @@ traverse_kernel(const TraverseParams prm) {
     }
 
     for (long long wi = blockIdx.x; wi < nwork; wi += gridDim.x) {
-      const int b = (int)(wi / ngroups), grp = (int)(wi % ngroups);
+      int b, grp;
+      if (listed) {                // the last partition whose work starts at or before wi
+          int lo_b = 0, hi_b = prm.num_parts;
+          while (hi_b - lo_b > 1) {
+              const int mid = (lo_b + hi_b) >> 1;
+              if ((long long)__ldg(prm.wl_offs + mid) <= wi) lo_b = mid; else hi_b = mid;
+          }
+          b = lo_b;
+          grp = __ldg(prm.wl_list + (size_t)b * prm.wl_stride + (int)(wi - __ldg(prm.wl_offs + b)));
+      } else { b = (int)(wi / ngroups); grp = (int)(wi % ngroups); }
       const long long lo = (long long)b * prm.ppb;
       const int n = (int)min((long long)prm.ppb, (long long)N - lo);
       int ndense = 0;

@@ -1,0 +1,111 @@
+"""Queries that leave out partitions by distance bounds (csrc/distance_bounds.cuh, csrc/prune.cuh) against the sequential restatement: neighbour ids and distance bits
+must not depend on what was left out.  Sizes sit on the edges of the 256-row and 128-query tiles, of the
+32-coordinate stages and of the 32-row chunks in which groups may begin and end; rows that
+a tensor map cannot describe (dim not a multiple of 4, a base that is not 16-byte aligned) take the variant with
+ordinary loads."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle
+from tests import cases
+
+pytestmark = pytest.mark.gpu
+
+#        rows, dim, queries, parts, L, S, T, k, max_cand, distribution
+SIZES = [(2048, 32, 128, 8, 2, 4, 10, 10, 100, "latent"),      # everything a multiple of its tile
+         (2049, 33, 129, 8, 2, 4, 10, 10, 30, "latent"),       # one beyond every tile; plain loads
+         (2047, 31, 127, 7, 2, 3, 7, 5, 20, "latent"),
+         (640, 64, 1, 2, 1, 5, 10, 1, 10, "latent"),           # one query, two partitions
+         (13000, 96, 300, 200, 2, 5, 5, 3, 15, "mixture"),     # partitions of 65: several in one tile, one beyond two chunks
+         (20000, 128, 260, 5, 2, 6, 10, 40, 200, "unit"),      # concentrated distances: little can be left out
+         (9001, 50, 77, 9, 3, 5, 7, 13, 130, "mixture"),       # 200-byte rows
+         (4000, 960, 20, 4, 2, 4, 10, 10, 60, "unit"),
+         (6000, 24, 140, 30, 2, 4, 1, 7, 40, "latent"),        # windows of one point
+         (3000, 16, 50, 6, 2, 4, 10, 600, 900, "latent")]      # lists longer than a partition
+
+
+def _rows(rng, n, dim, dist):
+    if dist == "mixture":
+        return cases.mixture(rng, n, dim, centres=20)
+    if dist == "unit":
+        return cases.unit_uniform(rng, n, dim)
+    return cases.latent_linear(rng, n, max(2, dim // 4), dim, 0.01)
+
+
+def _bits(t):
+    return t.cpu().numpy().view(np.uint32)
+
+
+def _check(data, query, L, S, P, T, k, mc, proj, shift=0):
+    from dciknn_cuda_b200 import DCI
+    dim = data.shape[1]
+    o = oracle.OracleDCI(dim, L, S, P, T, proj)
+    o.add(data)
+    oi, od = o.query(query, k, 5000, mc)
+    store = torch.empty(data.size + 16, device="cuda")
+    d = store[shift:shift + data.size].view(data.shape)
+    d.copy_(torch.from_numpy(data))
+    g = DCI(dim, L, S, P, T, proj=torch.from_numpy(proj))
+    g.add(d)
+    q = torch.from_numpy(query).cuda()
+    for mode in (1, 0, 2):
+        g.set_pruning(mode)
+        ids, dists = g.query(q, k, 5000, max_num_candidates=mc, return_int_ids=True)
+        assert np.array_equal(ids.cpu().numpy(), oi), mode
+        assert np.array_equal(_bits(dists), od.view(np.uint32)), mode
+        packed = g.query_packed(q, k, 5000, max_num_candidates=mc)
+        assert torch.equal(packed & 0xFFFFFFFF, ids.to(torch.int64) & 0xFFFFFFFF), mode
+    for mode in (1, 0):
+        g.set_pruning(mode)
+        ids, dists = torch.empty_like(ids), torch.empty_like(dists)
+        g.query_noalloc(q, ids, dists, 5000, max_num_candidates=mc)
+        assert np.array_equal(ids.cpu().numpy(), oi) and np.array_equal(_bits(dists), od.view(np.uint32)), mode
+
+
+@pytest.mark.parametrize("size", SIZES, ids=lambda s: "%dx%d_q%d" % s[:3])
+def test_answers_do_not_depend_on_what_is_left_out(size):
+    n, dim, nq, P, L, S, T, k, mc, dist = size
+    rng = np.random.default_rng(n + dim)
+    z = _rows(rng, n + nq, dim, dist)
+    _check(np.ascontiguousarray(z[:n]), np.ascontiguousarray(z[n:]), L, S, P, T, k, mc, cases.unit_rows(rng, L * S, dim))
+
+
+@pytest.mark.parametrize("kind", ["unaligned", "sorted", "duplicates", "huge", "tiny", "far", "nan"])
+def test_answers_do_not_depend_on_what_is_left_out_for_unusual_rows(kind):
+    rng, mc = np.random.default_rng(5), 60
+    n, dim, nq = 3000, 32, 40
+    z = _rows(rng, n + nq, dim, "latent")
+    data, query = z[:n].copy(), z[n:].copy()
+    if kind == "sorted":            # near rows in few partitions
+        data = data[np.argsort(data[:, 0], kind="stable")].copy()
+    elif kind == "duplicates":      # equal distances across partitions, ties by id
+        data[n // 2:] = data[:n // 2]
+        query[:20] = data[:20]
+    elif kind == "huge":            # squared norms beyond the range in which bounds are formed, some beyond fp32
+        data[::7] *= np.float32(1e16)
+        data[3::50] *= np.float32(1e19)
+        query[::5] *= np.float32(1e16)
+    elif kind == "tiny":            # squares that underflow
+        data *= np.float32(1e-21)
+        query *= np.float32(1e-21)
+    elif kind == "far":
+        query *= np.float32(1000)
+    elif kind == "nan":             # queries and rows without distances beside ordinary ones
+        query[3] = np.nan
+        data[70:90, 5] = np.nan
+    proj = cases.unit_rows(rng, 8, dim)
+    if kind in ("nan", "huge"):     # compared with the call that traverses every pair
+        from dciknn_cuda_b200 import DCI
+        g = DCI(dim, 2, 4, 6, 10, proj=torch.from_numpy(proj))
+        g.add(torch.from_numpy(data).cuda())
+        q = torch.from_numpy(query).cuda()
+        out = []
+        for mode in (2, 1, 0):
+            g.set_pruning(mode)
+            ids, dists = g.query(q, 10, 5000, max_num_candidates=mc, return_int_ids=True)
+            out.append((ids.cpu(), dists.cpu().view(torch.int32)))
+        for o in out[1:]:
+            assert torch.equal(out[0][0], o[0]) and torch.equal(out[0][1], o[1])
+        return
+    _check(data, query, 2, 4, 6, 10, 10, mc, proj, shift=1 if kind == "unaligned" else 0)
