@@ -27,6 +27,7 @@
 #include "distance_bounds.cuh"
 #include "prune.cuh"
 #include "traverse.cuh"
+#include "exhaustive.cuh"
 
 namespace {
 
@@ -486,6 +487,129 @@ int traverse_pruned(dci_b200 *h, dci::TraverseParams prm, int first, unsigned ch
     return 0;
 }
 
+// Whether the stop rule can fire in no partition, whatever the keys, so that every point is a candidate.
+// The rule ends a traversal after iteration min(max(a, outer * S - 1), max(a, c), n * S * T - 1) where a and c are
+// the k-th and max_cand-th smallest promotion iterations of lane-0 points (c absent when there are fewer).
+// Iterations run to at most wcap - 1, so the first term is harmless when outer * S >= wcap; with max_cand >= n
+// either c is absent or every point is a lane-0 point and c is the last promotion of all; the third term counts
+// more iterations than there are windows when n * T >= ceil(n / T) + 2.
+bool always_exhaustive(const dci::TraverseParams &prm) {
+    if (prm.max_cand < prm.ppb || prm.max_cand <= prm.knn || prm.outer_s < prm.wcap) return false;
+    const long long last = (long long)prm.N - (long long)(prm.num_parts - 1) * prm.ppb;
+    for (long long n : {(long long)prm.ppb, last})
+        if (n * prm.T < (n + prm.T - 1) / prm.T + 2) return false;
+    return true;
+}
+
+// How an exhaustive call is answered (exhaustive.cuh).
+struct ExactPlan {
+    int mode = 0;                 // 0: by the traversal, 1: exact_scan_kernel, 2: nearest_groups_kernel
+    int batch = 0;                // queries per launch
+    int tile = 1, slices = 1, slice_rows = 0, threads = 0, topk_cap = 0;
+    int group_rows = 0, num_groups = 0, first = 0;
+    size_t smem = 0, bytes = 0;   // dynamic shared memory; working memory (mode 1: lists, mode 2: bounds and a flag)
+};
+
+// Sizes alone decide.  The scan does two packed operations per query and coordinate pair: about 9 coordinates of
+// 10^6 rows x queries per microsecond on the whole chip; the groups read all rows once, multiply them with the
+// padded queries (as in prune_first_round) and work out about twice `first` groups per query.
+ExactPlan plan_exact(const dci_b200 *h, const dci::TraverseParams &prm, int num_queries, size_t avail) {
+    ExactPlan p;
+    if (prm.blind || prm.work_stats || prm.phase_cycles || h->pruning == 2 || prm.knn > dci::kMaxTopK || prm.dim > 4096 ||
+        !always_exhaustive(prm))
+        return p;
+    const double cells = (double)prm.N * prm.dim;
+    const size_t smem_max = h->smem_optin - 12 * 1024;       // beside the kernels' static arrays
+    p.mode = 1;
+    p.batch = num_queries;
+    p.threads = dci::kScanThreads;
+    p.topk_cap = next_pow2(prm.knn + p.threads);
+    p.tile = num_queries >= 8 * h->sm_count ? 8 : (num_queries >= 4 ? 4 : 1);
+    while (p.tile > 1 && (size_t)p.tile * ((size_t)p.topk_cap * 16 + (size_t)prm.dim * 4) > smem_max) p.tile = p.tile == 8 ? 4 : 1;
+    p.smem = (size_t)p.tile * ((size_t)p.topk_cap * 16 + (size_t)prm.dim * 4);
+    const int tiles = (num_queries + p.tile - 1) / p.tile;
+    // slices of at least four rows per thread, until there are two CTAs per SM
+    p.slices = std::max(1, std::min((2 * h->sm_count + tiles - 1) / tiles, prm.N / (4 * p.threads)));
+    p.slice_rows = (prm.N + p.slices - 1) / p.slices;
+    p.slices = (prm.N + p.slice_rows - 1) / p.slice_rows;
+    p.bytes = p.slices > 1 ? sizeof(uint64_t) * (size_t)num_queries * p.slices * prm.knn : 0;
+    if (p.bytes > avail || p.bytes > ((size_t)1 << 30)) { p.slices = 1; p.slice_rows = prm.N; p.bytes = 0; }
+
+    ExactPlan g = p;
+    g.mode = 2;
+    g.threads = dci::kNgThreads;
+    g.topk_cap = next_pow2(prm.knn + dci::kNgThreads);
+    g.smem = (size_t)g.topk_cap * 16 + (size_t)prm.dim * 4;
+    g.group_rows = 64;
+    while (prm.N / g.group_rows > 16384) g.group_rows *= 2;
+    g.num_groups = (prm.N + g.group_rows - 1) / g.group_rows;
+    g.first = prm.knn + 4;
+    const size_t per_query = sizeof(uint32_t) * (size_t)g.num_groups;
+    g.batch = (int)std::min<size_t>((size_t)num_queries, (std::min<size_t>(avail, (size_t)256 << 20) - 512) / per_query);
+    g.bytes = per_query * g.batch + 512;
+    if (g.num_groups < 2 * g.first || g.batch < 1 || (g.batch < num_queries && g.batch < 1024)) return p;
+    if (h->pruning == 1) return g;
+    if (g.num_groups < 8 * g.first) return p;
+    const double scan_us = cells * num_queries / 9.0e6;
+    const double padded = (double)((num_queries + dci::kLbQueries - 1) / dci::kLbQueries) * dci::kLbQueries;
+    const double groups_us = std::max(cells * 4.0 / 6.0e6, cells * padded * 2.0 / 0.35e9) + 30.0 +
+                             2.0 * num_queries * g.first * g.group_rows * prm.dim * 4.0 / 2.5e6;
+    return scan_us > 1.5 * groups_us ? g : p;
+}
+
+// ws: plan.bytes of working memory.
+int launch_exact(dci_b200 *h, const ExactPlan &plan, const dci::TraverseParams &prm, const float *d_query, int num_queries,
+                 unsigned char *ws, int *d_ids, float *d_dists, unsigned long long *d_packed, cudaStream_t st) {
+    for (int q0 = 0; q0 < num_queries; q0 += plan.batch) {
+        dci::ExactParams e;
+        memset(&e, 0, sizeof(e));
+        e.data = prm.data; e.query = d_query + (size_t)q0 * prm.dim;
+        e.n = prm.N; e.dim = prm.dim; e.nq = std::min(plan.batch, num_queries - q0); e.knn = prm.knn; e.topk_cap = plan.topk_cap;
+        e.vec4 = prm.dim % 4 == 0 && ((uintptr_t)prm.data & 15) == 0;
+        e.vec8 = prm.vec8;
+        e.slices = plan.slices; e.slice_rows = plan.slice_rows;
+        e.lists = (uint64_t *)ws;
+        e.out_ids = d_ids ? d_ids + (size_t)q0 * prm.knn : nullptr;
+        e.out_dists = d_dists ? d_dists + (size_t)q0 * prm.knn : nullptr;
+        e.out_packed = d_packed ? reinterpret_cast<uint64_t *>(d_packed) + (size_t)q0 * prm.knn : nullptr;
+        if (plan.mode == 2) {
+            // the flag word lies behind the bounds
+            const size_t lb_bytes = sizeof(uint32_t) * (size_t)plan.num_groups * e.nq;
+            int *failed = (int *)(ws + ((lb_bytes + 255) & ~(size_t)255));
+            DCI_CUDA(cudaMemsetAsync(ws, 0xFF, lb_bytes, st));
+            DCI_CUDA(cudaMemsetAsync(failed, 0, sizeof(int), st));
+            dci::TraverseParams bp = prm;
+            bp.query = d_query; bp.q0 = q0; bp.nq = e.nq;
+            if (int rc = launch_bounds(h, bp, plan.group_rows, plan.num_groups, (uint32_t *)ws, failed, st)) return rc;
+            e.lb = (const uint32_t *)ws; e.failed = failed;
+            e.num_groups = plan.num_groups; e.group_rows = plan.group_rows; e.first = plan.first;
+            e.keep = (float)dci::bounds_keep(prm.dim);
+            DCI_CUDA(cudaFuncSetAttribute(dci::nearest_groups_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
+            dci::nearest_groups_kernel<<<e.nq, plan.threads, plan.smem, st>>>(e);
+            h->launches++;
+            DCI_CUDA(cudaGetLastError());
+            continue;
+        }
+        auto go = [&](auto kern) -> int {
+            DCI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
+            kern<<<dim3((e.nq + plan.tile - 1) / plan.tile, plan.slices), plan.threads, plan.smem, st>>>(e);
+            h->launches++;
+            DCI_CUDA(cudaGetLastError());
+            return 0;
+        };
+        if (int rc = plan.tile == 8 ? go(dci::exact_scan_kernel<8>) : (plan.tile == 4 ? go(dci::exact_scan_kernel<4>) : go(dci::exact_scan_kernel<1>)))
+            return rc;
+        if (plan.slices > 1) {
+            const int merge_threads = 256, merge_cap = next_pow2(prm.knn + merge_threads);
+            dci::merge_partitions_kernel<<<e.nq, merge_threads, (size_t)merge_cap * 16, st>>>(
+                e.lists, plan.slices, prm.knn, prm.knn, merge_cap, 0, e.nq, nullptr, e.out_ids, e.out_dists, 0, e.out_packed);
+            h->launches++;
+            DCI_CUDA(cudaGetLastError());
+        }
+    }
+    return 0;
+}
+
 int check_handle(dci_b200 *h) {
     if (!h) return fail(DCI_B200_ERR_ARG, "null handle");
     return 0;
@@ -805,6 +929,20 @@ static int query_impl(dci_b200_t *h, const float *d_query, int num_queries, int 
         DCI_CUDA(cudaMemsetAsync(h->stats.p, 0, bytes, st));
         prm.work_stats = (long long *)h->stats.p;
         h->stats_nq = num_queries;
+    }
+    const ExactPlan exact = plan_exact(h, prm, num_queries, ~(size_t)0);
+    if (exact.mode) {      // no index entry is looked at: neither projections nor a traversal
+        DCI_CUDA(h->prune.ensure(exact.bytes));
+        if (timing) { DCI_CUDA(cudaEventRecord(h->ev[2], st)); }
+        if (int rc = launch_exact(h, exact, prm, d_query, num_queries, (unsigned char *)h->prune.p, d_ids, d_dists, d_packed, st)) return rc;
+        h->last_qbatch = 1;
+        if (timing) {
+            DCI_CUDA(cudaEventRecord(h->ev[3], st));
+            DCI_CUDA(cudaEventSynchronize(h->ev[3]));
+            DCI_CUDA(cudaEventElapsedTime(&h->t_traverse, h->ev[2], h->ev[3]));
+            h->t_traverse_launches = 1;
+        }
+        return 0;
     }
     DCI_CUDA(h->qproj.ensure(sizeof(float) * (size_t)I * num_queries));
     prm.qproj = (const float *)h->qproj.p;
@@ -1407,6 +1545,8 @@ int query_noalloc_impl(dci_b200 *h, dci::TraverseParams prm, int nthreads, unsig
         return fail(DCI_B200_ERR_UNSUPPORTED,
                     "this index and k need %zu bytes of working memory, the built-in scratch of the allocation-free query holds %u",
                     slabs + per_query + 256 + ((size_t)DCI_B200_NOALLOC_SCRATCH_BYTES - avail), (unsigned)DCI_B200_NOALLOC_SCRATCH_BYTES);
+    const ExactPlan exact = plan_exact(h, prm, num_queries, avail);
+    if (exact.mode) return launch_exact(h, exact, prm, prm.query, num_queries, scratch, d_ids, d_dists, nullptr, st);
     // the handle's own flag word and timing events are created on first use, so neither is used here
     if (int rc = launch_project(h, prm.query, num_queries, const_cast<float *>(prm.qproj), st, flag_word, false)) return rc;
     const int batch = (int)std::min<size_t>((size_t)num_queries, (avail - slabs - 256) / per_query);

@@ -1,7 +1,8 @@
 // Lower bounds of the distances between all queries and groups of consecutive rows, on the 5th-generation
 // tensor cores.  A group is a partition of the index (pruning: a partition whose nearest row is provably
-// farther than the k-th candidate found so far cannot change a query's answer, so it is not traversed).
-// No value computed here reaches a result: every returned distance is the fixed fp32 chain of the traversal.
+// farther than the k-th candidate found so far cannot change a query's answer, so it is not traversed), or a
+// run of 64 or more rows (exhaustive queries).  No value computed here reaches a result: every returned
+// distance is the fixed fp32 chain of the traversal.
 //
 // For query q and group g the kernel produces
 //     v[g][q] = min over rows x of the group of  keep * |x|^2 - 2 <x, q>~

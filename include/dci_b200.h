@@ -216,8 +216,9 @@ long long dci_b200_device_alloc_calls(void);
  * row, so tests reach whatever a CTA keeps from one pair to the next. */
 int dci_b200_set_max_ctas(dci_b200_t *h, int max_ctas);
 
-/* Whether queries leave out partitions that provably cannot change their answer, being beyond the candidates
- * already known (dciknn_cuda_b200/csrc/prune.cuh).  0, the default, where the sizes of the call make it pay; 1 wherever it is possible;
+/* Whether queries leave out what provably cannot change their answer: partitions beyond the candidates already
+ * known (dciknn_cuda_b200/csrc/prune.cuh), or the whole traversal where every point is a candidate
+ * (csrc/exhaustive.cuh).  0, the default, where the sizes of the call make it pay; 1 wherever it is possible;
  * 2 never.  Results are the same, bit for bit.  A diagnostic, for tests and comparisons. */
 int dci_b200_set_pruning(dci_b200_t *h, int mode);
 

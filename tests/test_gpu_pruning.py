@@ -1,6 +1,7 @@
-"""Queries that leave out partitions by distance bounds (csrc/distance_bounds.cuh, csrc/prune.cuh) against the sequential restatement: neighbour ids and distance bits
+"""Queries that leave out work by distance bounds (csrc/distance_bounds.cuh, csrc/prune.cuh) or answer an exhaustive
+call without the index (csrc/exhaustive.cuh) against the sequential restatement: neighbour ids and distance bits
 must not depend on what was left out.  Sizes sit on the edges of the 256-row and 128-query tiles, of the
-32-coordinate stages and of the 32-row chunks in which groups may begin and end; rows that
+32-coordinate stages, of the 32-row chunks in which groups may begin and end and of the 512-thread scan; rows that
 a tensor map cannot describe (dim not a multiple of 4, a base that is not 16-byte aligned) take the variant with
 ordinary loads."""
 import numpy as np
@@ -22,7 +23,15 @@ SIZES = [(2048, 32, 128, 8, 2, 4, 10, 10, 100, "latent"),      # everything a mu
          (9001, 50, 77, 9, 3, 5, 7, 13, 130, "mixture"),       # 200-byte rows
          (4000, 960, 20, 4, 2, 4, 10, 10, 60, "unit"),
          (6000, 24, 140, 30, 2, 4, 1, 7, 40, "latent"),        # windows of one point
-         (3000, 16, 50, 6, 2, 4, 10, 600, 900, "latent")]      # lists longer than a partition
+         (3000, 16, 50, 6, 2, 4, 10, 600, 900, "latent"),      # lists longer than a partition
+         # every point a candidate
+         (2000, 100, 500, 100, 2, 7, 10, 10, 100, "latent"),
+         (2000, 100, 1, 100, 2, 7, 10, 10, 100, "latent"),
+         (511, 37, 3, 3, 1, 4, 10, 10, 1000, "latent"),        # fewer rows than threads
+         (8193, 8, 1185, 10, 1, 2, 16, 1, 900, "mixture"),     # tiles of eight queries, one of them short
+         (8192, 64, 129, 7, 2, 3, 7, 128, 1280, "unit"),
+         (4097, 12, 40, 5, 2, 3, 10, 300, 3000, "latent"),
+         (6000, 960, 9, 4, 1, 3, 10, 10, 10000, "unit")]
 
 
 def _rows(rng, n, dim, dist):
@@ -71,9 +80,10 @@ def test_answers_do_not_depend_on_what_is_left_out(size):
     _check(np.ascontiguousarray(z[:n]), np.ascontiguousarray(z[n:]), L, S, P, T, k, mc, cases.unit_rows(rng, L * S, dim))
 
 
+@pytest.mark.parametrize("mc", [60, 3000])      # the traversal's quota, or every point a candidate
 @pytest.mark.parametrize("kind", ["unaligned", "sorted", "duplicates", "huge", "tiny", "far", "nan"])
-def test_answers_do_not_depend_on_what_is_left_out_for_unusual_rows(kind):
-    rng, mc = np.random.default_rng(5), 60
+def test_answers_do_not_depend_on_what_is_left_out_for_unusual_rows(kind, mc):
+    rng = np.random.default_rng(5)
     n, dim, nq = 3000, 32, 40
     z = _rows(rng, n + nq, dim, "latent")
     data, query = z[:n].copy(), z[n:].copy()
