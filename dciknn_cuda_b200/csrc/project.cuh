@@ -115,4 +115,83 @@ project_exact_kernel(const float *__restrict__ x, long long n, int dim,
     }
 }
 
+// Few points: the kernel above gives 256 points to a CTA, so a query batch ran on a handful of SMs and took as long
+// as one CTA needs for its tile (20 us for up to 256 queries x 128 coordinates x 20 directions; 1 000 points in 4 CTAs).
+// Here a CTA has 32 points and a thread one direction of four of them: per four coordinates four 128-bit broadcast
+// reads of the points and four reads of the direction (rows padded to an odd stride, so the lanes' directions lie on
+// different banks) feed sixteen multiply-adds.  The next 64 coordinates are copied (cp.async) while these are added.
+// Bound by the latency of those copies; the same chain per key, hence the same bits.
+constexpr int kPsmRows = 32, kPsmK = 64, kPsmXPad = 68, kPsmPPad = 65, kPsmMaxIndices = 48;
+
+__host__ __device__ inline size_t psm_buffer_floats(int num_indices) {      // a multiple of 4: the points' rows are read as float4
+    return (size_t)kPsmRows * kPsmXPad + (((size_t)num_indices * kPsmPPad + 3) & ~(size_t)3);
+}
+
+__global__ void __launch_bounds__(kPsmMaxIndices * 8)
+project_small_kernel(const float *__restrict__ x, long long n, int dim, const float *__restrict__ proj, int num_indices,
+                     float *__restrict__ out) {
+    extern __shared__ __align__(16) float psm_smem[];
+    const int tid = threadIdx.x;
+    const long long p0 = (long long)blockIdx.x * kPsmRows;
+    const int rows = (int)min((long long)kPsmRows, n - p0);
+    const size_t buf = psm_buffer_floats(num_indices);
+    auto load = [&](int k0, float *xs) {
+        auto copy = [](float *dst, const float *src, bool live) {      // 4 bytes, zero when not live
+            const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(live ? 4 : 0) : "memory");
+        };
+        float *ps = xs + kPsmRows * kPsmXPad;
+        for (int e = tid; e < rows * kPsmK; e += blockDim.x) {
+            const int r = e / kPsmK, k = e % kPsmK;
+            const bool live = k0 + k < dim;
+            copy(xs + r * kPsmXPad + k, x + (p0 + r) * dim + (live ? k0 + k : 0), live);
+        }
+        for (int e = tid; e < num_indices * kPsmK; e += blockDim.x) {
+            const int d = e / kPsmK, k = e % kPsmK;
+            const bool live = k0 + k < dim;
+            copy(ps + d * kPsmPPad + k, proj + (size_t)d * dim + (live ? k0 + k : 0), live);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int d = tid % num_indices, r0 = tid / num_indices * 4;
+    const bool active = r0 < rows;
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    load(0, psm_smem);
+    for (int k0 = 0, c = 0; k0 < dim; k0 += kPsmK, ++c) {
+        if (k0 + kPsmK < dim) {
+            load(k0 + kPsmK, psm_smem + (size_t)((c + 1) & 1) * buf);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        if (active) {
+            const float *xs = psm_smem + (size_t)(c & 1) * buf;
+            const float *ps = xs + kPsmRows * kPsmXPad + d * kPsmPPad;
+            xs += r0 * kPsmXPad;
+            const int kn = min(kPsmK, (dim - k0 + 3) & ~3);         // coordinates beyond the row's end are zero
+#pragma unroll 4
+            for (int k = 0; k < kn; k += 4) {
+                float4 xv[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) xv[u] = *reinterpret_cast<const float4 *>(xs + u * kPsmXPad + k);
+                const float a = ps[k], b = ps[k + 1], e = ps[k + 2], f = ps[k + 3];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    acc[u] = __fmaf_rn(a, xv[u].x, acc[u]);
+                    acc[u] = __fmaf_rn(b, xv[u].y, acc[u]);
+                    acc[u] = __fmaf_rn(e, xv[u].z, acc[u]);
+                    acc[u] = __fmaf_rn(f, xv[u].w, acc[u]);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (active) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (r0 + u < rows) out[(size_t)d * n + p0 + r0 + u] = acc[u];
+    }
+}
+
 }  // namespace dci
