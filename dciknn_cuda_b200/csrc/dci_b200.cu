@@ -283,6 +283,15 @@ int launch_build(dci_b200 *h, const float *d_unsorted, cudaStream_t st) {
     const int I = h->L * h->S;
     const int nthreads = h->ppb >= 4096 ? 1024 : (h->ppb >= 1024 ? 512 : 256);
     const long long nseg = (long long)I * h->num_parts;
+    if (sizeof(ValT) == 2 && h->ppb <= 32) {
+        const unsigned grid = (unsigned)std::min<long long>((nseg + dci::kTinyWarps - 1) / dci::kTinyWarps, (long long)h->sm_count * 8);
+        dci::build_tiny_segments_kernel<<<grid, dci::kTinyWarps * 32, 0, st>>>(d_unsorted, h->num_points, I, h->ppb, h->num_parts,
+                                                                               (float *)h->keys.p, (int *)h->ids.p, (uint16_t *)h->pos.p,
+                                                                               (float *)h->keysT.p, h->T);
+        h->launches++;
+        DCI_CUDA(cudaGetLastError());
+        return 0;
+    }
     cudaFuncAttributes fa;
     DCI_CUDA(cudaFuncGetAttributes(&fa, dci::build_segments_kernel<ValT, true>));
     // the opt-in limit covers static + dynamic shared memory, and the driver reserves 1 KB per CTA
