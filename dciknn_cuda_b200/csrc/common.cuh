@@ -385,6 +385,48 @@ __device__ __forceinline__ void cta_select2(Get get, int cnt, int k1, int k2, in
     __syncthreads();
 }
 
+// A value with at least k (1 <= k <= cnt) of get(0..cnt) at or below it and, unless they lie very unevenly, few
+// more: one histogram of 128 to 256 equal ranges between the smallest and the largest.  A quarter of the work of
+// cta_select2, which finds the k-th itself.  sel, res as there.
+template <typename Get>
+__device__ __forceinline__ uint32_t cta_cover(Get get, int cnt, int k, uint32_t (*sel)[256], uint32_t *res) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    for (int i = tid; i < 256; i += blockDim.x) sel[0][i] = 0u;
+    if (tid == 0) { res[0] = 0xFFFFFFFFu; res[1] = 0u; }
+    __syncthreads();
+    uint32_t mn = 0xFFFFFFFFu, mx = 0u;
+    for (int j = tid; j < cnt; j += blockDim.x) { const uint32_t v = get(j); mn = min(mn, v); mx = max(mx, v); }
+    mn = __reduce_min_sync(0xFFFFFFFFu, mn);
+    mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+    if (lane == 0) { atomicMin(&res[0], mn); atomicMax(&res[1], mx); }
+    __syncthreads();
+    mn = res[0];
+    const int shift = max(0, 24 - __clz(res[1] - mn));        // (max - min) >> shift is below 256
+    for (int j = tid; j < cnt; j += blockDim.x) atomicAdd(&sel[0][(get(j) - mn) >> shift], 1u);
+    __syncthreads();
+    if (tid < 32) {
+        uint32_t c[8], sum = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { c[j] = sel[0][lane * 8 + j]; sum += c[j]; }
+        uint32_t inc = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        const int owner = __ffs(__ballot_sync(0xFFFFFFFFu, inc >= (uint32_t)k)) - 1;
+        if (lane == owner) {
+            uint32_t before = inc - sum;
+            int d = 0;
+            while (d < 7 && before + c[d] < (uint32_t)k) { before += c[d]; ++d; }
+            const uint64_t end = (uint64_t)mn + ((uint64_t)(lane * 8 + d + 1) << shift) - 1;      // last value of the range
+            res[2] = end > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)end;
+        }
+    }
+    __syncthreads();
+    return res[2];
+}
+
 // In-place ascending bitonic sort of `len` (power of two) u64 keys in shared
 // memory by the whole CTA.  Ends with a barrier.
 __device__ __forceinline__ void cta_bitonic_sort_u64(uint64_t *a, int len) {
@@ -420,9 +462,9 @@ __device__ __forceinline__ int warp_append_slot(bool pred, int *counter) {
 // Usage: init; every round all threads call offer with at most one key each
 // (kEmptySlot for none); finish leaves the k smallest, ascending, in
 // result()[0..k) (padded with kEmptySlot).
-// When the buffer fills up it is reduced to the k smallest: the k-th smallest
-// distance is found by radix selection, the few keys not above it are moved to
-// the other half and only those are sorted.
+// When the buffer fills up it is reduced to the k smallest: a distance that at
+// least k keys do not exceed is found (cta_cover), the few keys not above it are
+// moved to the other half and only those are sorted.
 struct CtaTopK {
     uint64_t *buf, *other;
     int *count;
@@ -441,23 +483,26 @@ struct CtaTopK {
     __device__ __forceinline__ void compact() {   // all threads; keeps the k smallest, sorted
         int c = *count;
         __syncthreads();
-        if (c > k && c > 128) {       // a short list is cheaper to sort outright
-            uint32_t tau[2];
+        // a short list is cheaper to sort outright; a long one is narrowed first (values that fall into one range
+        // of the histogram stop the narrowing, and the sort takes them all)
+        while (c > 128 && c > k + (k >> 2)) {
             const uint64_t *src = buf;
-            cta_select2([src](int j) { return (uint32_t)(src[j] >> 32); }, c, k, k, 32, sel, res, tau);
+            const uint32_t tau = cta_cover([src](int j) { return (uint32_t)(src[j] >> 32); }, c, k, sel, res);
             if (threadIdx.x == 0) *count = 0;
             __syncthreads();
             for (int j0 = 0; j0 < c; j0 += blockDim.x) {
                 const int j = j0 + threadIdx.x;
                 const uint64_t key = j < c ? buf[j] : kEmptySlot;
-                const bool take = j < c && (uint32_t)(key >> 32) <= tau[0];
+                const bool take = j < c && (uint32_t)(key >> 32) <= tau;
                 const int sl = warp_append_slot(take, count);
                 if (take) other[sl] = key;
             }
             __syncthreads();
-            c = *count;
+            const int kept = *count;
             uint64_t *t = buf; buf = other; other = t;
             __syncthreads();
+            if (kept == c) break;
+            c = kept;
         }
         int len = 2;
         while (len < c) len <<= 1;

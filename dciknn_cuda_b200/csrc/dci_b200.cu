@@ -632,6 +632,15 @@ int launch_exact(dci_b200 *h, const ExactPlan &plan, const dci::TraverseParams &
     return 0;
 }
 
+// Entries of a merge's selection buffer: room for all lists of a query, so that they are narrowed once (12 -> 8 us for
+// one query of 100 lists), as long as the CTAs of the call are few; 32 KB of buffers per CTA cost a large call more
+// than they save (1 000 queries: 14 -> 19 us).
+int merge_capacity(const dci_b200 *h, int num_queries, int lists, int list_len, int width, int threads) {
+    const int least = next_pow2(width + threads);
+    if (num_queries > 4 * h->sm_count || (long long)lists * list_len + threads > 2048) return least;
+    return std::max(least, next_pow2(lists * list_len + threads));
+}
+
 int check_handle(dci_b200 *h) {
     if (!h) return fail(DCI_B200_ERR_ARG, "null handle");
     return 0;
@@ -936,7 +945,8 @@ static int query_impl(dci_b200_t *h, const float *d_query, int num_queries, int 
     // while it selects, and the shared buffers would overlay them
     prm.topk_global = (prm.topk_cap > 2048 || blind) ? 1 : 0;
     const int merge_threads = 256;
-    const int merge_cap = next_pow2(out_width + merge_threads);
+    // room for all lists of a query where that fits, so that they are narrowed once
+    const int merge_cap = merge_capacity(h, num_queries, h->num_parts, prm.kpart, out_width, merge_threads);
     const bool merge_global = merge_cap > 2048;
 
     if (h->stats_on & 2) {
@@ -1583,7 +1593,7 @@ int query_noalloc_impl(dci_b200 *h, dci::TraverseParams prm, int nthreads, unsig
                            ? (uint32_t *)(scratch + slabs + align256(sizeof(uint64_t) * (size_t)prm.num_parts * prm.kpart * batch))
                            : nullptr;
     const int merge_threads = 256;
-    const int merge_cap = next_pow2(prm.knn + merge_threads);
+    const int merge_cap = merge_capacity(h, num_queries, prm.num_parts, prm.kpart, prm.knn, merge_threads);
     // the same kernel instances as the regular query
     const bool lean = !prm.blind && !prm.topk_global && prm.vec8 && !prm.work_stats && !prm.phase_cycles && prm.T > 1;
     void (*kern)(const dci::TraverseParams) =
