@@ -509,6 +509,15 @@ int traverse_pruned(dci_b200 *h, dci::TraverseParams prm, int first, unsigned ch
     return 0;
 }
 
+// Entries of a merge's selection buffer: room for all lists of a query, so that they are narrowed once (12 -> 8 us for
+// one query of 100 lists), as long as the CTAs of the call are few; 32 KB of buffers per CTA cost a large call more
+// than they save (1 000 queries: 14 -> 19 us).
+int merge_capacity(const dci_b200 *h, int num_queries, int lists, int list_len, int width, int threads) {
+    const int least = next_pow2(width + threads);
+    if (num_queries > 4 * h->sm_count || (long long)lists * list_len + threads > 2048) return least;
+    return std::max(least, next_pow2(lists * list_len + threads));
+}
+
 // Whether the stop rule can fire in no partition, whatever the keys, so that every point is a candidate.
 // The rule ends a traversal after iteration min(max(a, outer * S - 1), max(a, c), n * S * T - 1) where a and c are
 // the k-th and max_cand-th smallest promotion iterations of lane-0 points (c absent when there are fewer).
@@ -527,31 +536,29 @@ bool always_exhaustive(const dci::TraverseParams &prm) {
 struct ExactPlan {
     int mode = 0;                 // 0: by the traversal, 1: exact_scan_kernel, 2: nearest_groups_kernel
     int batch = 0;                // queries per launch
-    int tile = 1, slices = 1, slice_rows = 0, threads = 0, topk_cap = 0;
+    int slices = 1, slice_rows = 0, threads = 0, topk_cap = 0;
     int group_rows = 0, num_groups = 0, first = 0;
     size_t smem = 0, bytes = 0;   // dynamic shared memory; working memory (mode 1: lists, mode 2: bounds and a flag)
 };
 
-// Sizes alone decide.  The scan does two packed operations per query and coordinate pair: about 9 coordinates of
-// 10^6 rows x queries per microsecond on the whole chip; the groups read all rows once, multiply them with the
-// padded queries (as in prune_first_round) and work out about twice `first` groups per query.
+// Sizes alone decide.  The scan reads every row once per query (5 TB/s out of L2); the groups read all rows once,
+// multiply them with the padded queries (as in prune_first_round), take two launches more, and one CTA per query then
+// works out about twice `first` groups (40 GB/s each).  Measured with 128 coordinates and k = 10 (us a call): 10 000
+// rows, 8 queries: scan 34, groups 40; 100 queries: 103 and 40; 256 coordinates, k = 100, 100 000 rows, 2 queries: 114
+// and 209; 1 000 queries: 4 663 and 1 214.
 ExactPlan plan_exact(const dci_b200 *h, const dci::TraverseParams &prm, int num_queries, size_t avail) {
     ExactPlan p;
     if (prm.blind || prm.work_stats || prm.phase_cycles || h->pruning == 2 || prm.knn > dci::kMaxTopK || prm.dim > 4096 ||
         !always_exhaustive(prm))
         return p;
     const double cells = (double)prm.N * prm.dim;
-    const size_t smem_max = h->smem_optin - 12 * 1024;       // beside the kernels' static arrays
     p.mode = 1;
     p.batch = num_queries;
     p.threads = dci::kScanThreads;
     p.topk_cap = next_pow2(prm.knn + p.threads);
-    p.tile = num_queries >= 8 * h->sm_count ? 8 : (num_queries >= 4 ? 4 : 1);
-    while (p.tile > 1 && (size_t)p.tile * ((size_t)p.topk_cap * 16 + (size_t)prm.dim * 4) > smem_max) p.tile = p.tile == 8 ? 4 : 1;
-    p.smem = (size_t)p.tile * ((size_t)p.topk_cap * 16 + (size_t)prm.dim * 4);
-    const int tiles = (num_queries + p.tile - 1) / p.tile;
-    // slices of at least four rows per thread, until there are two CTAs per SM
-    p.slices = std::max(1, std::min((2 * h->sm_count + tiles - 1) / tiles, prm.N / (4 * p.threads)));
+    p.smem = (size_t)p.topk_cap * 16 + (size_t)prm.dim * 4;
+    // slices of at least one row per thread, until every SM has a CTA
+    p.slices = std::max(1, std::min((h->sm_count + num_queries - 1) / num_queries, prm.N / p.threads));
     p.slice_rows = (prm.N + p.slices - 1) / p.slices;
     p.slices = (prm.N + p.slice_rows - 1) / p.slice_rows;
     p.bytes = p.slices > 1 ? sizeof(uint64_t) * (size_t)num_queries * p.slices * prm.knn : 0;
@@ -562,8 +569,8 @@ ExactPlan plan_exact(const dci_b200 *h, const dci::TraverseParams &prm, int num_
     g.threads = dci::kNgThreads;
     g.topk_cap = next_pow2(prm.knn + dci::kNgThreads);
     g.smem = (size_t)g.topk_cap * 16 + (size_t)prm.dim * 4;
-    g.group_rows = 64;
-    while (prm.N / g.group_rows > 16384) g.group_rows *= 2;
+    g.group_rows = 32;                                       // the bounds' epilogue takes minima of 32 rows at a time
+    while (prm.N / g.group_rows > 32768) g.group_rows *= 2;
     g.num_groups = (prm.N + g.group_rows - 1) / g.group_rows;
     g.first = prm.knn + 4;
     const size_t per_query = sizeof(uint32_t) * (size_t)g.num_groups;
@@ -572,11 +579,11 @@ ExactPlan plan_exact(const dci_b200 *h, const dci::TraverseParams &prm, int num_
     if (g.num_groups < 2 * g.first || g.batch < 1 || (g.batch < num_queries && g.batch < 1024)) return p;
     if (h->pruning == 1) return g;
     if (g.num_groups < 8 * g.first) return p;
-    const double scan_us = cells * num_queries / 9.0e6;
+    const double scan_us = 8.0 + cells * num_queries * 4.0 / 5.0e6;
     const double padded = (double)((num_queries + dci::kLbQueries - 1) / dci::kLbQueries) * dci::kLbQueries;
-    const double groups_us = std::max(cells * 4.0 / 6.0e6, cells * padded * 2.0 / 0.35e9) + 30.0 +
-                             2.0 * num_queries * g.first * g.group_rows * prm.dim * 4.0 / 2.5e6;
-    return scan_us > 1.5 * groups_us ? g : p;
+    const double groups_us = 28.0 + std::max(cells * 4.0 / 6.0e6, cells * padded * 2.0 / 0.35e9) +
+                             2.0 * g.first * g.group_rows * prm.dim * 4.0 / 4.0e4 * std::max(1.0, (double)num_queries / h->sm_count);
+    return scan_us > groups_us ? g : p;
 }
 
 // ws: plan.bytes of working memory.
@@ -612,17 +619,12 @@ int launch_exact(dci_b200 *h, const ExactPlan &plan, const dci::TraverseParams &
             DCI_CUDA(cudaGetLastError());
             continue;
         }
-        auto go = [&](auto kern) -> int {
-            DCI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
-            kern<<<dim3((e.nq + plan.tile - 1) / plan.tile, plan.slices), plan.threads, plan.smem, st>>>(e);
-            h->launches++;
-            DCI_CUDA(cudaGetLastError());
-            return 0;
-        };
-        if (int rc = plan.tile == 8 ? go(dci::exact_scan_kernel<8>) : (plan.tile == 4 ? go(dci::exact_scan_kernel<4>) : go(dci::exact_scan_kernel<1>)))
-            return rc;
+        DCI_CUDA(cudaFuncSetAttribute(dci::exact_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
+        dci::exact_scan_kernel<<<dim3(e.nq, plan.slices), plan.threads, plan.smem, st>>>(e);
+        h->launches++;
+        DCI_CUDA(cudaGetLastError());
         if (plan.slices > 1) {
-            const int merge_threads = 256, merge_cap = next_pow2(prm.knn + merge_threads);
+            const int merge_threads = 256, merge_cap = merge_capacity(h, e.nq, plan.slices, prm.knn, prm.knn, merge_threads);
             dci::merge_partitions_kernel<<<e.nq, merge_threads, (size_t)merge_cap * 16, st>>>(
                 e.lists, plan.slices, prm.knn, prm.knn, merge_cap, 0, e.nq, nullptr, e.out_ids, e.out_dists, 0, e.out_packed);
             h->launches++;
@@ -630,15 +632,6 @@ int launch_exact(dci_b200 *h, const ExactPlan &plan, const dci::TraverseParams &
         }
     }
     return 0;
-}
-
-// Entries of a merge's selection buffer: room for all lists of a query, so that they are narrowed once (12 -> 8 us for
-// one query of 100 lists), as long as the CTAs of the call are few; 32 KB of buffers per CTA cost a large call more
-// than they save (1 000 queries: 14 -> 19 us).
-int merge_capacity(const dci_b200 *h, int num_queries, int lists, int list_len, int width, int threads) {
-    const int least = next_pow2(width + threads);
-    if (num_queries > 4 * h->sm_count || (long long)lists * list_len + threads > 2048) return least;
-    return std::max(least, next_pow2(lists * list_len + threads));
 }
 
 int check_handle(dci_b200 *h) {

@@ -1,7 +1,7 @@
 // Queries whose stop rule provably never fires: every point of every partition is a candidate, so the answer is
 // the exact k nearest rows by (distance, id) and nothing of the index is needed.  Two ways to it, with the
 // distance chain of the traversal (ascending fma, IEEE square root), hence the same bits:
-//   exact_scan_kernel     every row against a tile of queries; for small problems and few queries
+//   exact_scan_kernel     every row, one query a CTA; for small problems and few queries
 //   nearest_groups_kernel for large ones: distance_bounds_kernel gives a lower bound for every (query, group of
 //                         rows); one CTA per query works out the groups with the smallest bounds, which gives a
 //                         k-th distance, and then only the groups whose bound does not exceed it.
@@ -15,7 +15,7 @@ struct ExactParams {
     const float *data, *query;      // query: first query of this launch
     int n, dim, nq, knn, topk_cap;  // topk_cap: power of two >= knn + blockDim.x
     int vec4, vec8;
-    int slice_rows, slices;         // exact_scan_kernel: rows per CTA, CTAs per query tile
+    int slice_rows, slices;         // exact_scan_kernel: rows per CTA, CTAs per query
     uint64_t *lists;                // slices > 1: [nq][slices][knn]
     int *out_ids;                   // slices == 1: the result itself, [nq][knn] ...
     float *out_dists;
@@ -36,101 +36,55 @@ __device__ __forceinline__ void write_result(const ExactParams &p, int q, const 
     }
 }
 
-// Squared distances of one row to QT queries whose coordinates lie coordinate-major in shared memory (qs[c * QT + t]).
-template <int QT>
-__device__ __forceinline__ void row_to_queries(const float *__restrict__ row, const float *qs, int dim, int vec4, int vec8,
-                                               float (&sq)[QT]) {
-#pragma unroll
-    for (int t = 0; t < QT; ++t) sq[t] = 0.0f;
-    auto one = [&](float x, const float *q) {
-        if constexpr (QT == 1) {
-            const float d = __fsub_rn(x, q[0]);
-            sq[0] = __fmaf_rn(d, d, sq[0]);
-        } else {
-            const float2 xx = make_float2(x, x);
-#pragma unroll
-            for (int t = 0; t < QT; t += 4) {
-                const float4 b = *reinterpret_cast<const float4 *>(q + t);
-                const float2 r0 = fma2sq(sub2(xx, make_float2(b.x, b.y)), make_float2(sq[t], sq[t + 1]));
-                const float2 r1 = fma2sq(sub2(xx, make_float2(b.z, b.w)), make_float2(sq[t + 2], sq[t + 3]));
-                sq[t] = r0.x; sq[t + 1] = r0.y; sq[t + 2] = r1.x; sq[t + 3] = r1.y;
+// Distances of the rows row_of(0 .. count) to the query in shared memory, offered to topk; rows beyond the k-th
+// distance known so far are abandoned.  All threads call; row_of may return a row >= p.n (none).
+template <typename RowOf>
+__device__ __forceinline__ void offer_rows(const ExactParams &p, const float *qv, CtaTopK &topk, int count, RowOf row_of) {
+    for (int base = 0; base < count; base += blockDim.x) {
+        const int j = base + threadIdx.x;
+        float bd = __int_as_float(0x7F800000), bsq = bd;
+        const uint64_t th = *topk.thresh;       // set at compactions only, the same for all threads here
+        if (th != kEmptySlot && (uint32_t)(th >> 32) < 0x7F7F7F7Fu) {
+            bd = __uint_as_float((uint32_t)(th >> 32));
+            const float up = __uint_as_float((uint32_t)(th >> 32) + 1u);
+            bsq = __fmul_ru(up, up);            // sq > bsq  =>  sqrt(sq) > bd
+        }
+        uint64_t key = kEmptySlot;
+        if (j < count) {
+            const long long r = row_of(j);
+            if (r < p.n) {
+                const float *row = p.data + (size_t)r * p.dim;
+                const float d = p.vec8 ? dist_sequential_v8(row, qv, p.dim, bsq) : dist_sequential(row, qv, p.dim, p.vec4);
+                if (d >= 0.0f && d <= bd) key = ((uint64_t)__float_as_uint(d) << 32) | (uint32_t)r;      // a NaN is no candidate
             }
         }
-    };
-    if (vec8) {
-#pragma unroll 2
-        for (int c = 0; c < dim; c += 8) {
-            float a[8];
-            ld_row8(row + c, a);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) one(a[e], qs + (size_t)(c + e) * QT);
-        }
-    } else if (vec4) {
-#pragma unroll 4
-        for (int c = 0; c < dim; c += 4) {
-            const float4 a = __ldg(reinterpret_cast<const float4 *>(row + c));
-            one(a.x, qs + (size_t)c * QT); one(a.y, qs + (size_t)(c + 1) * QT);
-            one(a.z, qs + (size_t)(c + 2) * QT); one(a.w, qs + (size_t)(c + 3) * QT);
-        }
-    } else {
-#pragma unroll 4
-        for (int c = 0; c < dim; ++c) one(__ldg(row + c), qs + (size_t)c * QT);
+        topk.offer(key);
     }
-}
-
-__device__ __forceinline__ uint64_t distance_key(float sq, uint32_t id) {      // a NaN is no candidate
-    const float d = __fsqrt_rn(sq);
-    return d >= 0.0f ? ((uint64_t)__float_as_uint(d) << 32) | id : kEmptySlot;
 }
 
 constexpr int kScanThreads = 512;
 
-// grid (query tiles, slices).  Dynamic shared memory: QT pairs of selection buffers | query coordinates.
-template <int QT>
+// grid (queries, slices).  Dynamic shared memory: selection buffers | query.  Tiles of four and eight queries per CTA,
+// which read a row once for all of them, were slower for the few queries this kernel is for: every offer of a row's
+// keys is a CTA-wide step per query (2 000 x 100 rows, 500 queries: 68 us with four, 97 us with eight).
 __global__ void __launch_bounds__(kScanThreads, 2)
 exact_scan_kernel(const ExactParams p) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     __shared__ uint32_t s_sel[2][256];
     __shared__ uint32_t s_res[4];
-    __shared__ TopKSlot s_slot[QT];
-    const int q0 = blockIdx.x * QT, tid = threadIdx.x;
-    uint64_t *bufs = reinterpret_cast<uint64_t *>(dyn_smem);
-    float *qs = reinterpret_cast<float *>(dyn_smem + (size_t)QT * p.topk_cap * 16);
-    for (int e = tid; e < p.dim * QT; e += blockDim.x) {
-        const int t = e / p.dim, c = e - t * p.dim;
-        qs[c * QT + t] = q0 + t < p.nq ? p.query[(size_t)(q0 + t) * p.dim + c] : 0.0f;
-    }
-    if (tid < QT) { s_slot[tid].count = 0; s_slot[tid].half = 0; s_slot[tid].thresh = kEmptySlot; }
-    __syncthreads();
+    __shared__ int s_count;
+    __shared__ uint64_t s_thresh;
+    const int q = blockIdx.x, tid = threadIdx.x;
+    float *qv = reinterpret_cast<float *>(dyn_smem + (size_t)p.topk_cap * 16);
+    for (int c = tid; c < p.dim; c += blockDim.x) qv[c] = p.query[(size_t)q * p.dim + c];
+    CtaTopK topk;
+    topk.init(reinterpret_cast<uint64_t *>(dyn_smem), &s_count, &s_thresh, s_sel, s_res, p.topk_cap, p.knn);
     const long long r0 = (long long)blockIdx.y * p.slice_rows;
-    const long long r1 = min((long long)p.n, r0 + p.slice_rows);
-    for (long long base = r0; base < r1; base += blockDim.x) {
-        const long long r = base + tid;
-        const bool live = r < r1;
-        float sq[QT];
-        row_to_queries<QT>(p.data + (size_t)(live ? r : r0) * p.dim, qs, p.dim, p.vec4, p.vec8, sq);
-#pragma unroll
-        for (int t = 0; t < QT; ++t) {
-            if (q0 + t < p.nq) {
-                uint64_t *mine = bufs + (size_t)t * 2 * p.topk_cap;
-                CtaTopK topk = topk_slot_open(&s_slot[t], mine, s_sel, s_res, p.topk_cap, p.knn);
-                topk.offer(live ? distance_key(sq[t], (uint32_t)r) : kEmptySlot);
-                topk_slot_close(&s_slot[t], topk, mine);
-            }
-        }
-    }
-    for (int t = 0; t < QT && q0 + t < p.nq; ++t) {
-        uint64_t *mine = bufs + (size_t)t * 2 * p.topk_cap;
-        CtaTopK topk = topk_slot_open(&s_slot[t], mine, s_sel, s_res, p.topk_cap, p.knn);
-        topk.finish();
-        const uint64_t *res = topk.result();
-        if (p.slices == 1) write_result(p, q0 + t, res);
-        else {
-            uint64_t *out = p.lists + ((size_t)(q0 + t) * p.slices + blockIdx.y) * p.knn;
-            for (int j = tid; j < p.knn; j += blockDim.x) out[j] = res[j];
-        }
-        __syncthreads();
-    }
+    offer_rows(p, qv, topk, (int)max(0ll, min((long long)p.n - r0, (long long)p.slice_rows)), [r0](int j) { return r0 + j; });
+    topk.finish();
+    if (p.slices == 1) { write_result(p, q, topk.result()); return; }
+    uint64_t *out = p.lists + ((size_t)q * p.slices + blockIdx.y) * p.knn;
+    for (int j = tid; j < p.knn; j += blockDim.x) out[j] = topk.result()[j];
 }
 
 constexpr int kNgThreads = 512;
@@ -172,29 +126,9 @@ nearest_groups_kernel(const ExactParams p) {
         cta_select2([lb, stride](int j) { return lb[(size_t)j * stride]; }, p.num_groups, p.first, p.first, 32, s_sel, s_res, out);
         first = out[0];
     }
-    // works out the listed groups; rows beyond the k-th distance so far are abandoned
     auto work = [&]() {
-        const int rows = s_listed * p.group_rows;
-        for (int base = 0; base < rows; base += blockDim.x) {
-            const int j = base + tid;
-            float bd = __int_as_float(0x7F800000), bsq = bd;
-            const uint64_t th = s_thresh;       // set at compactions only, the same for all threads here
-            if (th != kEmptySlot && (uint32_t)(th >> 32) < 0x7F7F7F7Fu) {
-                bd = __uint_as_float((uint32_t)(th >> 32));
-                const float up = __uint_as_float((uint32_t)(th >> 32) + 1u);
-                bsq = __fmul_ru(up, up);        // sq > bsq  =>  sqrt(sq) > bd
-            }
-            uint64_t key = kEmptySlot;
-            if (j < rows) {
-                const long long r = (long long)s_group[j / p.group_rows] * p.group_rows + j % p.group_rows;
-                if (r < p.n) {
-                    const float *row = p.data + (size_t)r * p.dim;
-                    const float d = p.vec8 ? dist_sequential_v8(row, qv, p.dim, bsq) : dist_sequential(row, qv, p.dim, p.vec4);
-                    if (d >= 0.0f && d <= bd) key = ((uint64_t)__float_as_uint(d) << 32) | (uint32_t)r;
-                }
-            }
-            topk.offer(key);
-        }
+        offer_rows(p, qv, topk, s_listed * p.group_rows,
+                   [&](int j) { return (long long)s_group[j / p.group_rows] * p.group_rows + j % p.group_rows; });
         __syncthreads();
         if (tid == 0) s_listed = 0;
         __syncthreads();

@@ -28,7 +28,7 @@ SIZES = [(2048, 32, 128, 8, 2, 4, 10, 10, 100, "latent"),      # everything a mu
          (2000, 100, 500, 100, 2, 7, 10, 10, 100, "latent"),
          (2000, 100, 1, 100, 2, 7, 10, 10, 100, "latent"),
          (511, 37, 3, 3, 1, 4, 10, 10, 1000, "latent"),        # fewer rows than threads
-         (8193, 8, 1185, 10, 1, 2, 16, 1, 900, "mixture"),     # tiles of eight queries, one of them short
+         (8193, 8, 1185, 10, 1, 2, 16, 1, 900, "mixture"),     # more queries than fit the scan
          (8192, 64, 129, 7, 2, 3, 7, 128, 1280, "unit"),
          (4097, 12, 40, 5, 2, 3, 10, 300, 3000, "latent"),
          (6000, 960, 9, 4, 1, 3, 10, 10, 10000, "unit")]
