@@ -345,8 +345,12 @@ int pick_buckets(dci_b200 *h, dci::TraverseParams &prm, int nthreads, size_t sta
     return std::min(std::max(prm.wcap / 2, 64), 16384);
 }
 
+// How a traversal runs: work arrays in shared memory or in a slab of device memory per CTA, CTAs per SM.
+struct TraverseGeometry { bool smem; size_t dyn, per_cta; int per_sm; };
+
+// Works the geometry out and sets what depends on it in prm (buckets, query groups, slab layout).
 template <typename ValT, typename PosT>
-int launch_traverse(dci_b200 *h, dci::TraverseParams prm, int nthreads, cudaStream_t st) {
+int plan_traverse(dci_b200 *h, dci::TraverseParams &prm, int nthreads, TraverseGeometry *geo) {
     cudaFuncAttributes fa;
     DCI_CUDA(cudaFuncGetAttributes(&fa, dci::traverse_kernel<ValT, PosT, true, true>));
     const size_t static_smem = fa.sharedSizeBytes;
@@ -365,7 +369,7 @@ int launch_traverse(dci_b200 *h, dci::TraverseParams prm, int nthreads, cudaStre
     // ... and pays off when work items are exhaustive: lane 0 of a partition sees about ppb / T
     // promotions, so a quota well above that (with an iteration cap beyond the last window) is never met
     prm.qbatch = 1;
-    const bool likely_exhaustive = !prm.wl_offs && (long long)prm.max_cand * prm.T * 2 > 3ll * prm.ppb && prm.outer_s >= prm.wcap;
+    const bool likely_exhaustive = (long long)prm.max_cand * prm.T * 2 > 3ll * prm.ppb && prm.outer_s >= prm.wcap;
     if (smem && prm.vec8 && !prm.topk_global && !prm.blind && likely_exhaustive) {
         prm.dense_cap = next_pow2(prm.kpart + nthreads / 4);
         // per query a pair of selection buffers; for the group the query vectors, always kMaxQBatch slots
@@ -378,6 +382,17 @@ int launch_traverse(dci_b200 *h, dci::TraverseParams prm, int nthreads, cudaStre
     prm.topk_global_off = lay.fallback_bytes + (smem ? 0 : lay.big_bytes);
     const size_t per_cta = prm.topk_global_off + (prm.topk_global ? (size_t)prm.topk_cap * 16 : 0);
     const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(h->smem_per_sm / (dyn + static_smem + 1024), 2048 / nthreads));
+    *geo = {smem, dyn, per_cta, per_sm};
+    return 0;
+}
+
+template <typename ValT, typename PosT>
+int launch_traverse(dci_b200 *h, dci::TraverseParams prm, int nthreads, cudaStream_t st) {
+    TraverseGeometry geo;
+    if (int rc = plan_traverse<ValT, PosT>(h, prm, nthreads, &geo)) return rc;
+    const bool smem = geo.smem;
+    const size_t dyn = geo.dyn, per_cta = geo.per_cta;
+    const int per_sm = geo.per_sm;
     h->last_qbatch = prm.qbatch;
     const long long nwork = (long long)((prm.nq + prm.qbatch - 1) / prm.qbatch) * prm.num_parts;
     unsigned grid = (unsigned)std::min<long long>(nwork, (long long)h->sm_count * per_sm);
@@ -410,7 +425,7 @@ int launch_traverse(dci_b200 *h, dci::TraverseParams prm, int nthreads, cudaStre
 // 128); a pair that need not be traversed saves about 0.31 ns of one SM per point and simple index (62 us for
 // 10 000 points x 20 indices), and k nearest rows spread evenly over P partitions leave
 // P * (1 - exp(-k / P)) of them to visit.  The factor 2 covers the small launches in between and the last
-// waves of the two rounds.
+// waves of the rounds.
 int prune_first_round(const dci_b200 *h, const dci::TraverseParams &prm, int num_queries) {
     if (prm.blind || prm.work_stats || prm.phase_cycles || !h->distance_bound || h->pruning == 2) return 0;
     if (prm.num_parts < 2 || prm.ppb < 64) return 0;
@@ -425,7 +440,8 @@ int prune_first_round(const dci_b200 *h, const dci::TraverseParams &prm, int num
 }
 
 // Working memory of a pruned batch, in 256-byte pieces: bounds | round-1 cut-offs | work lists | offsets |
-// [counters of both rounds | tickets | failure flag] (the bracketed part starts as zeros).
+// [counters of the rounds | tickets | failure flag] (the bracketed part starts as zeros).
+constexpr int kMaxRounds = 4;
 struct PruneSpace {
     size_t lb, thresh, list, offs, zero, bytes;
     int zero_words;
@@ -434,10 +450,10 @@ struct PruneSpace {
         PruneSpace s;
         s.lb = 0;
         s.thresh = s.lb + up(sizeof(uint32_t) * (size_t)parts * nq);
-        s.list = s.thresh + up(sizeof(uint32_t) * (size_t)nq);
+        s.list = s.thresh + up(sizeof(uint32_t) * (size_t)nq * (kMaxRounds - 1));
         s.offs = s.list + up(sizeof(int) * (size_t)parts * nq);
         s.zero = s.offs + up(sizeof(int) * ((size_t)parts + 1));
-        s.zero_words = 2 * parts + 3;
+        s.zero_words = kMaxRounds * parts + kMaxRounds + 1;
         s.bytes = s.zero + up(sizeof(int) * (size_t)s.zero_words);
         return s;
     }
@@ -474,10 +490,21 @@ int launch_bounds(dci_b200 *h, const dci::TraverseParams &prm, int group_rows, i
     return tma ? go(dci::distance_bounds_kernel<false>) : go(dci::distance_bounds_kernel<true>);
 }
 
-// One batch with pruning: bounds, then the two rounds.  traverse(prm) launches the traversal of prm's work list.
+// One batch with pruning: bounds, then the rounds.  traverse(prm) launches the traversal of prm's work list.
 // ws: PruneSpace::make(num_parts, nq).bytes of device memory; prm.qbound and prm.part_topk are set.
+// per_item: queries that a traversal CTA takes together; resident: CTAs that run at the same time.
 template <typename Traverse>
-int traverse_pruned(dci_b200 *h, dci::TraverseParams prm, int first, unsigned char *ws, cudaStream_t st, Traverse traverse) {
+int traverse_pruned(dci_b200 *h, dci::TraverseParams prm, int first, int per_item, long long resident, unsigned char *ws,
+                    cudaStream_t st, Traverse traverse) {
+    // Few pairs: round 1 fills its last wave of CTAs, which costs nothing and leaves less to round 2.  (Rounding down
+    // does not pay: with fewer than k partitions the k-th candidate is loose, and round 2 grew by more than the wave.)
+    const double waves = (double)prm.nq * first / ((double)resident * per_item);
+    if (waves < 4.0)
+        first = std::max(first, std::min(prm.num_parts - 1, (int)(ceil(waves) * resident * per_item / prm.nq)));
+    // Many pairs: further rounds of a quarter of the first each, since every round brings the k-th candidate down.
+    // Each costs a last wave of CTAs: 67 waves of 1.25M x 96 lose 1 % with one round more, 675 waves of 1M x 128 go from
+    // 71 to 52 ms with two.
+    const int rounds = waves < 16.0 ? 2 : (waves < 200.0 ? 3 : 4);
     const PruneSpace sp = PruneSpace::make(prm.num_parts, prm.nq);
     uint32_t *lb = (uint32_t *)(ws + sp.lb);
     int *zero = (int *)(ws + sp.zero);
@@ -488,20 +515,23 @@ int traverse_pruned(dci_b200 *h, dci::TraverseParams prm, int first, unsigned ch
     DCI_CUDA(cudaGetLastError());
     dci::SelectParams s;
     memset(&s, 0, sizeof(s));
-    int *failed = zero + 2 * prm.num_parts + 2;
+    int *failed = zero + kMaxRounds * prm.num_parts + kMaxRounds;
     if (int rc = launch_bounds(h, prm, prm.ppb, prm.num_parts, lb, failed, st)) return rc;
     s.lb = lb; s.failed = failed;
     s.query = prm.query + (size_t)prm.q0 * prm.dim;
     s.part_topk = prm.part_topk; s.thresh = (uint32_t *)(ws + sp.thresh); s.qbound = prm.qbound;
     s.offs = (int *)(ws + sp.offs); s.list = (int *)(ws + sp.list);
-    s.nq = prm.nq; s.num_groups = prm.num_parts; s.q_stride = prm.nq; s.first = first; s.knn = prm.knn; s.kpart = prm.kpart;
+    s.nq = prm.nq; s.num_groups = prm.num_parts; s.q_stride = prm.nq; s.first = first; s.step = std::max(1, first / 4); s.knn = prm.knn; s.kpart = prm.kpart;
+    s.per_item = per_item;
     s.dim = prm.dim; s.keep = (float)dci::bounds_keep(prm.dim);
     prm.wl_offs = s.offs; prm.wl_list = s.list; prm.wl_stride = prm.nq;
-    for (int round = 1; round <= 2; ++round) {
+    for (int round = 1; round <= rounds; ++round) {
         s.cnt = zero + (round - 1) * prm.num_parts;
-        s.ticket = zero + 2 * prm.num_parts + (round - 1);
-        if (round == 1) dci::select_work_kernel<1><<<prm.nq, 128, 0, st>>>(s);
-        else dci::select_work_kernel<2><<<prm.nq, 128, 0, st>>>(s);
+        s.ticket = zero + kMaxRounds * prm.num_parts + (round - 1);
+        s.round = round; s.last = round == rounds;
+        prm.wl_cnt = s.cnt;
+        if (round == 1) dci::select_work_kernel<true><<<prm.nq, 128, 0, st>>>(s);
+        else dci::select_work_kernel<false><<<prm.nq, 128, 0, st>>>(s);
         h->launches++;
         DCI_CUDA(cudaGetLastError());
         if (int rc = traverse(prm)) return rc;
@@ -1013,7 +1043,18 @@ static int query_impl(dci_b200_t *h, const float *d_query, int num_queries, int 
                 return p.wcap <= 65535 ? launch_traverse<uint16_t, uint16_t>(h, p, nthreads, st)
                                        : launch_traverse<uint32_t, uint16_t>(h, p, nthreads, st);
             };
-            rc = prune_first ? traverse_pruned(h, prm, prune_first, (unsigned char *)h->prune.p, st, traverse) : traverse(prm);
+            if (prune_first) {
+                dci::TraverseParams p = prm;
+                TraverseGeometry geo;
+                rc = !pos16(p.ppb, h->T) ? plan_traverse<uint32_t, uint32_t>(h, p, nthreads, &geo)
+                                         : (p.wcap <= 65535 ? plan_traverse<uint16_t, uint16_t>(h, p, nthreads, &geo)
+                                                            : plan_traverse<uint32_t, uint16_t>(h, p, nthreads, &geo));
+                if (!rc)
+                    rc = traverse_pruned(h, prm, prune_first, p.qbatch, (long long)h->sm_count * geo.per_sm, (unsigned char *)h->prune.p,
+                                         st, traverse);
+            } else {
+                rc = traverse(prm);
+            }
         }
         if (rc) return rc;
         if (timing) DCI_CUDA(cudaEventRecord(h->ev[3], st));
@@ -1607,7 +1648,7 @@ int query_noalloc_impl(dci_b200 *h, dci::TraverseParams prm, int nthreads, unsig
             DCI_CUDA(cudaGetLastError());
             return 0;
         };
-        if (int rc = prune_first ? traverse_pruned(h, prm, prune_first, scratch + lists_end, st, traverse) : traverse(prm)) return rc;
+        if (int rc = prune_first ? traverse_pruned(h, prm, prune_first, 1, (long long)h->sm_count * per_sm, scratch + lists_end, st, traverse) : traverse(prm)) return rc;
         dci::merge_partitions_kernel<<<prm.nq, merge_threads, (size_t)merge_cap * 16, st>>>(
             prm.part_topk, prm.num_parts, prm.kpart, prm.knn, merge_cap, q0, prm.nq, nullptr, d_ids, d_dists, 0);
         h->launches++;

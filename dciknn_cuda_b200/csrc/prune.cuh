@@ -2,12 +2,15 @@
 //
 // Only a query's k nearest candidates over all partitions reach its result, so a partition whose nearest row
 // lies strictly beyond k candidates that are already known cannot change the answer.  distance_bounds_kernel
-// gives a rigorous lower bound of the nearest row of every partition; the pairs are then traversed in two
-// rounds.  Round 1: per query the partitions with the smallest bounds, about as many as hold the k nearest
-// rows when rows are spread evenly.  Round 2: every other partition whose bound does not exceed the k-th best
-// candidate of round 1 -- all of them when round 1 found fewer than k.  A pair that is left out keeps an empty
-// list.  Nothing is assumed about the data: clustered rows only make the lists shorter, and a distribution on
-// which the index finds few near neighbours (a loose k-th candidate) makes round 2 traverse more.
+// gives a rigorous lower bound of the nearest row of every partition; the pairs are then traversed in rounds.
+// Round 1: per query the partitions with the smallest bounds, about as many as hold the k nearest rows when rows
+// are spread evenly.  Every later round: of the remaining partitions those whose bound does not exceed the k-th best
+// candidate so far -- all of them when fewer than k were found --, in the last round all of these, in a round before
+// it only those with the next smallest bounds.  A pair that is left out keeps an empty list.  Nothing is assumed about
+// the data: clustered rows only make the lists shorter, and a distribution on which the index finds few near
+// neighbours (a loose k-th candidate) makes the last round traverse more.
+// 1M x 128, 10 000 queries, k = 10, 100 partitions (398 ms when every pair is traversed): two rounds with 8, 10, 12 and
+// 15 partitions first 145, 71, 60 and 73 ms; the rounds of a quarter each make that choice matter less.
 #pragma once
 #include "common.cuh"
 
@@ -18,11 +21,14 @@ struct SelectParams {
     const int *failed;            // not 0: the bounds are unusable, every pair is traversed in round 1
     const float *query;           // rows q0 .. of the call's queries
     uint64_t *part_topk;          // [nq][num_groups][kpart], empty lists where nothing was traversed
-    uint32_t *thresh;             // [nq] round 1's cut-off
+    uint32_t *thresh;             // [3][nq] largest bound of each round before the last, as found in round 1
     uint32_t *qbound;             // [nq] the shared distance bound of the traversal
     int *cnt, *offs, *list;       // [num_groups] (starts as 0), [num_groups + 1], [num_groups][q_stride]
     int *ticket;                  // starts as 0
-    int nq, num_groups, q_stride, first, knn, kpart, dim;
+    int nq, num_groups, q_stride, knn, kpart, dim;
+    int first, step;              // partitions of round 1, and at most of each later round but the last
+    int round, last;              // 1, 2, ..; last: 1 in the last round
+    int per_item;                 // queries of a partition that a traversal CTA takes together: offs counts such items
     float keep;
 };
 
@@ -38,7 +44,7 @@ __global__ void prune_init_kernel(uint4 *topk, size_t topk16, uint32_t *lb, size
 
 // One CTA per query.  Appends the query to the work lists of the partitions it has to visit in this round; the
 // last CTA to finish turns the list lengths into offsets.
-template <int ROUND>
+template <bool FIRST>
 __global__ void __launch_bounds__(128) select_work_kernel(const SelectParams p) {
     __shared__ uint32_t s_sel[2][256];
     __shared__ uint32_t s_res[4];
@@ -48,20 +54,24 @@ __global__ void __launch_bounds__(128) select_work_kernel(const SelectParams p) 
     const int q = blockIdx.x, tid = threadIdx.x;
     const uint32_t *lb = p.lb + q;
     const size_t stride = (size_t)p.q_stride;
-    uint32_t lo = 0u;                 // bounds above lo (ROUND 2) ...
+    uint32_t lo = 0u;                 // later rounds: bounds above lo ...
     float limit = __int_as_float(0x7F800000);      // ... and not beyond limit are taken
-    uint32_t hi = 0xFFFFFFFFu;        // ROUND 1: bounds up to hi are taken
-    if (ROUND == 1) {
+    uint32_t hi = 0xFFFFFFFFu;        // bounds up to hi are taken
+    if (FIRST) {
+        uint32_t cut[4] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu};
         if (!*p.failed && p.first < p.num_groups) {
-            uint32_t out[2];
-            cta_select2([lb, stride](int j) { return lb[(size_t)j * stride]; }, p.num_groups, p.first, p.first, 32, s_sel, s_res, out);
-            hi = out[0];
+            auto get = [lb, stride](int j) { return lb[(size_t)j * stride]; };
+            cta_select2(get, p.num_groups, p.first, min(p.first + p.step, p.num_groups), 32, s_sel, s_res, cut);
+            cta_select2(get, p.num_groups, min(p.first + 2 * p.step, p.num_groups), min(p.first + 2 * p.step, p.num_groups), 32,
+                        s_sel, s_res, cut + 2);
+            hi = cut[0];
         }
-        if (tid == 0) p.thresh[q] = hi;
+        if (tid < 3) p.thresh[(size_t)tid * p.nq + q] = tid == 0 ? cut[0] : (tid == 1 ? cut[1] : cut[2]);
     } else {
-        lo = p.thresh[q];
+        lo = p.thresh[(size_t)(p.round - 2) * p.nq + q];
+        if (!p.last) hi = p.thresh[(size_t)(p.round - 1) * p.nq + q];
         if (lo != 0xFFFFFFFFu) {      // the same for every thread
-            // k-th best candidate of round 1
+            // k-th best candidate so far
             const uint64_t *lists = p.part_topk + (size_t)q * p.num_groups * p.kpart;
             const int total = p.num_groups * p.kpart;
             uint32_t kth = 0xFFFFFFFFu;
@@ -87,10 +97,10 @@ __global__ void __launch_bounds__(128) select_work_kernel(const SelectParams p) 
             }
         }
     }
-    if (ROUND == 1 || lo != 0xFFFFFFFFu) {
+    if (FIRST || lo != 0xFFFFFFFFu) {
         for (int g = tid; g < p.num_groups; g += blockDim.x) {
             const uint32_t v = lb[(size_t)g * stride];
-            const bool take = ROUND == 1 ? v <= hi : (v > lo && !(ordered_to_float(v) > limit));
+            const bool take = v <= hi && (FIRST || (v > lo && !(ordered_to_float(v) > limit)));
             if (take) p.list[(size_t)g * stride + atomicAdd(p.cnt + g, 1)] = q;
         }
     }
@@ -104,7 +114,7 @@ __global__ void __launch_bounds__(128) select_work_kernel(const SelectParams p) 
         int run = 0;
         for (int g0 = 0; g0 < p.num_groups; g0 += blockDim.x) {
             const int g = g0 + tid, lane = tid & 31;
-            const int c = g < p.num_groups ? __ldcg(p.cnt + g) : 0;
+            const int c = g < p.num_groups ? (__ldcg(p.cnt + g) + p.per_item - 1) / p.per_item : 0;
             int inc = c;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {

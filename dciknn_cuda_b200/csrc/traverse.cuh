@@ -72,7 +72,8 @@ struct TraverseParams {
     uint32_t *qbound;          // nullptr or [nq]: per query of this launch, fp32 bits of an upper bound of its k-th
                                // smallest distance found so far (any partition); candidates beyond it are dropped
     const int *wl_offs;        // nullptr (every pair), or the pairs to traverse: offsets [num_parts + 1] into ...
-    const int *wl_list;        // ... the queries of each partition, [num_parts][wl_stride] (prune.cuh)
+    const int *wl_list;        // ... the queries of each partition, [num_parts][wl_stride], wl_cnt[b] of them; offsets
+    const int *wl_cnt;         // count groups of qbatch queries (prune.cuh)
     int wl_stride;
     int blind;                 // 1: no distances; a promoted point's key is its promotion iteration (needs topk_global)
     FastDiv divT;
@@ -394,7 +395,7 @@ traverse_kernel(const TraverseParams prm) {
     // deferred and their distances computed in one pass that loads each row once for all of them.
     const int Q = BATCH ? (prm.qbatch > 0 ? prm.qbatch : 1) : 1;
     const int ngroups = (prm.nq + Q - 1) / Q;
-    const bool listed = !BATCH && prm.wl_offs != nullptr;
+    const bool listed = prm.wl_offs != nullptr;
     const long long nwork = listed ? (long long)prm.wl_offs[prm.num_parts] : (long long)ngroups * prm.num_parts;
     long long t_last = 0;
 #define DCI_PHASE_MARK(slot_)                                                             \
@@ -413,14 +414,18 @@ traverse_kernel(const TraverseParams prm) {
               if ((long long)__ldg(prm.wl_offs + mid) <= wi) lo_b = mid; else hi_b = mid;
           }
           b = lo_b;
-          grp = __ldg(prm.wl_list + (size_t)b * prm.wl_stride + (int)(wi - __ldg(prm.wl_offs + b)));
+          grp = (int)(wi - __ldg(prm.wl_offs + b));
+          if (!BATCH) grp = __ldg(prm.wl_list + (size_t)b * prm.wl_stride + grp);      // one query: the work item itself
       } else { b = (int)(wi / ngroups); grp = (int)(wi % ngroups); }
       const long long lo = (long long)b * prm.ppb;
       const int n = (int)min((long long)prm.ppb, (long long)N - lo);
       int ndense = 0;
       for (int jq = 0; jq < Q; ++jq) {
-        const int ql = grp * Q + jq;
-        if (ql >= prm.nq) break;
+        int ql = grp * Q + jq;
+        if (BATCH && listed) {
+            if (ql >= __ldg(prm.wl_cnt + b)) break;
+            ql = __ldg(prm.wl_list + (size_t)b * prm.wl_stride + ql);
+        } else if (ql >= prm.nq) break;
         const int q = prm.q0 + ql;
         if (f_phase_cycles && tid == 0) t_last = clock64();
 
