@@ -345,6 +345,11 @@ int pick_buckets(dci_b200 *h, dci::TraverseParams &prm, int nthreads, size_t sta
     return std::min(std::max(prm.wcap / 2, 64), 16384);
 }
 
+// CTAs of the traversal kernels per SM: shared memory, threads, and 64 registers a thread.
+int traverse_ctas_per_sm(const dci_b200 *h, size_t smem, int nthreads) {
+    return (int)std::max<size_t>(1, std::min<size_t>(h->smem_per_sm / (smem + 1024), 1024 / nthreads));
+}
+
 // How a traversal runs: work arrays in shared memory or in a slab of device memory per CTA, CTAs per SM.
 struct TraverseGeometry { bool smem; size_t dyn, per_cta; int per_sm; };
 
@@ -381,7 +386,7 @@ int plan_traverse(dci_b200 *h, dci::TraverseParams &prm, int nthreads, TraverseG
     }
     prm.topk_global_off = lay.fallback_bytes + (smem ? 0 : lay.big_bytes);
     const size_t per_cta = prm.topk_global_off + (prm.topk_global ? (size_t)prm.topk_cap * 16 : 0);
-    const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(h->smem_per_sm / (dyn + static_smem + 1024), 2048 / nthreads));
+    const int per_sm = traverse_ctas_per_sm(h, dyn + static_smem, nthreads);
     *geo = {smem, dyn, per_cta, per_sm};
     return 0;
 }
@@ -499,12 +504,12 @@ int traverse_pruned(dci_b200 *h, dci::TraverseParams prm, int first, int per_ite
     // Few pairs: round 1 fills its last wave of CTAs, which costs nothing and leaves less to round 2.  (Rounding down
     // does not pay: with fewer than k partitions the k-th candidate is loose, and round 2 grew by more than the wave.)
     const double waves = (double)prm.nq * first / ((double)resident * per_item);
-    if (waves < 4.0)
+    if (waves < 16.0)
         first = std::max(first, std::min(prm.num_parts - 1, (int)(ceil(waves) * resident * per_item / prm.nq)));
     // Many pairs: further rounds of a quarter of the first each, since every round brings the k-th candidate down.
-    // Each costs a last wave of CTAs: 67 waves of 1.25M x 96 lose 1 % with one round more, 675 waves of 1M x 128 go from
-    // 71 to 52 ms with two.
-    const int rounds = waves < 16.0 ? 2 : (waves < 200.0 ? 3 : 4);
+    // Each costs a last wave of CTAs: 67 waves of 1.25M x 96 and 29 of 100k x 50 lose 2 % with one round more, 675 waves of
+    // 1M x 128 go from 71 to 52 ms with two.
+    const int rounds = waves < 100.0 ? 2 : (waves < 300.0 ? 3 : 4);
     const PruneSpace sp = PruneSpace::make(prm.num_parts, prm.nq);
     uint32_t *lb = (uint32_t *)(ws + sp.lb);
     int *zero = (int *)(ws + sp.zero);
@@ -608,7 +613,7 @@ ExactPlan plan_exact(const dci_b200 *h, const dci::TraverseParams &prm, int num_
     g.bytes = per_query * g.batch + 512;
     if (g.num_groups < 2 * g.first || g.batch < 1 || (g.batch < num_queries && g.batch < 1024)) return p;
     if (h->pruning == 1) return g;
-    if (g.num_groups < 8 * g.first) return p;
+    if (g.num_groups < 4 * g.first) return p;
     const double scan_us = 8.0 + cells * num_queries * 4.0 / 5.0e6;
     const double padded = (double)((num_queries + dci::kLbQueries - 1) / dci::kLbQueries) * dci::kLbQueries;
     const double groups_us = 28.0 + std::max(cells * 4.0 / 6.0e6, cells * padded * 2.0 / 0.35e9) +
@@ -1601,9 +1606,13 @@ int query_noalloc_impl(dci_b200 *h, dci::TraverseParams prm, int nthreads, unsig
     if (!smem) lay = dci::TraverseLayout<ValT>::make(nthreads, prm.dim, prm.topk_cap, prm.L, prm.wcap, prm.ppb, prm.nbuckets, false, prm.bkey != 0);
     const size_t dyn = smem ? lay.fixed_bytes + lay.big_bytes : lay.fixed_bytes;
     const size_t per_cta = align256(lay.fallback_bytes + (smem ? 0 : lay.big_bytes));
-    const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(h->smem_per_sm / (dyn + static_smem + 1024), 2048 / nthreads));
+    // the slabs set aside (and with them what is refused) count CTAs without regard to registers; the grid is what an
+    // SM really holds
+    const int slabs_per_sm = (int)std::max<size_t>(1, std::min<size_t>(h->smem_per_sm / (dyn + static_smem + 1024), 2048 / nthreads));
+    const int per_sm = std::min(slabs_per_sm, traverse_ctas_per_sm(h, dyn + static_smem, nthreads));
+    const long long slab_count = std::min<long long>((long long)num_queries * prm.num_parts, (long long)h->sm_count * slabs_per_sm);
     const long long max_grid = std::min<long long>((long long)num_queries * prm.num_parts, (long long)h->sm_count * per_sm);
-    const size_t slabs = per_cta * (size_t)max_grid;
+    const size_t slabs = per_cta * (size_t)slab_count;
     // per query of a pass: its per-partition result lists and its word of the shared distance bound
     const size_t per_query = sizeof(uint64_t) * (size_t)prm.num_parts * prm.kpart + sizeof(uint32_t);
     int prune_first = prune_first_round(h, prm, num_queries);
