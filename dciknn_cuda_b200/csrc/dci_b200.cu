@@ -472,7 +472,6 @@ int launch_bounds(dci_b200 *h, const dci::TraverseParams &prm, int group_rows, i
     bp.data = prm.data; bp.query = prm.query + (size_t)prm.q0 * prm.dim;
     bp.n = prm.N; bp.dim = prm.dim; bp.nq = prm.nq;
     bp.group_rows = group_rows; bp.num_groups = num_groups; bp.q_stride = prm.nq;
-    bp.keep = (float)dci::bounds_keep(prm.dim);
     bp.out = lb; bp.failed = failed;
     // units of one tile of rows and as many query tiles as leave about four units per SM
     const int row_tiles = (prm.N + dci::kLbRows - 1) / dci::kLbRows, q_tiles = (prm.nq + dci::kLbQueries - 1) / dci::kLbQueries;
@@ -528,7 +527,7 @@ int traverse_pruned(dci_b200 *h, dci::TraverseParams prm, int first, int per_ite
     s.offs = (int *)(ws + sp.offs); s.list = (int *)(ws + sp.list);
     s.nq = prm.nq; s.num_groups = prm.num_parts; s.q_stride = prm.nq; s.first = first; s.step = std::max(1, first / 4); s.knn = prm.knn; s.kpart = prm.kpart;
     s.per_item = per_item;
-    s.dim = prm.dim; s.keep = (float)dci::bounds_keep(prm.dim);
+    s.dim = prm.dim;
     prm.wl_offs = s.offs; prm.wl_list = s.list; prm.wl_stride = prm.nq;
     for (int round = 1; round <= rounds; ++round) {
         s.cnt = zero + (round - 1) * prm.num_parts;
@@ -647,7 +646,6 @@ int launch_exact(dci_b200 *h, const ExactPlan &plan, const dci::TraverseParams &
             if (int rc = launch_bounds(h, bp, plan.group_rows, plan.num_groups, (uint32_t *)ws, failed, st)) return rc;
             e.lb = (const uint32_t *)ws; e.failed = failed;
             e.num_groups = plan.num_groups; e.group_rows = plan.group_rows; e.first = plan.first;
-            e.keep = (float)dci::bounds_keep(prm.dim);
             DCI_CUDA(cudaFuncSetAttribute(dci::nearest_groups_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
             dci::nearest_groups_kernel<<<e.nq, plan.threads, plan.smem, st>>>(e);
             h->launches++;

@@ -5,13 +5,20 @@
 // distance is the fixed fp32 chain of the traversal.
 //
 // For query q and group g the kernel produces
-//     v[g][q] = min over rows x of the group of  keep * |x|^2 - 2 <x, q>~
-// where <x, q>~ is the tf32 inner product (fp32 rows read as they lie, the tensor core drops the low 13
-// mantissa bits).  keep * |q|^2 + v[g][q] is a lower bound of every squared distance of the group:
-//     | <x,q>~ - <x,q> | <= e |x||q|,   e = 2^-9 (two truncated operands) + dim * 2^-20 (accumulation),
-//     |x - q|^2 >= |x|^2 + |q|^2 - 2 <x,q>~ - 2 e |x||q| >= (1 - e) (|x|^2 + |q|^2) - 2 <x,q>~,
-// and keep (bounds_keep) is 1 - e less the rounding of the norms and of the sum itself.  Rows whose squared
-// norm exceeds 1e30 count as -inf (never pruned); rows with a NaN have no distance and are ignored.
+//     v[g][q] = min over rows x of the group of  row_term(x) - 2 s^2 <x~, q~>
+// where x~, q~ are the tf32 values that the tensor core makes of fp32 operands (it ignores the low 13 mantissa
+// bits: truncation) and s undoes the mean loss of that.  With x' = s x~, q' = s q~ and the residuals dx = x - x',
+// dq = q - q',
+//     <x, q> = <x', q'> + <dx, q> + <x', dq>,   so   | <x, q> - s^2 <x~, q~> | <= |dx||q| + |x'||dq|,
+// and for any r > 0:  2 |dx||q| <= |dx|^2 / r + r |q|^2,  2 |x'||dq| <= r |x'|^2 + |dq|^2 / r.  Hence
+//     |x - q|^2 = |x|^2 + |q|^2 - 2 <x, q>  >=  v + query_term(q)
+//     row_term(x) = keep |x|^2 - |dx|^2 / r,   query_term(q) = keep |q|^2 - |dq|^2 / r,
+// keep = 1 - r (with |x'| <= (1 + 2^-9) |x|) less the accumulation of the products (dim * 2^-22 of |x||q|; the MMAs add
+// eight products a step in fp32) and the rounding of the norms and of the sums.  The residuals are computed, not
+// bounded: about 0.2 * 2^-10 of the norm for mantissas without a pattern, which is what r is set to, against the 2^-9
+// of both operands' largest truncation (1.25M x 96 mixture, |x| about ten times the distances between neighbours,
+// 1 000 queries: 10.1 -> 6.9 ms).  Rows whose squared norm exceeds 1e30 count as -inf (never pruned); rows with a NaN
+// have no distance and are ignored.
 //
 // One persistent CTA per SM, warp-specialised like project_tf32x3_persistent_kernel: tiles of 128 queries x
 // 256 rows, 32 coordinates a stage (48 KB), four stages, accumulators double buffered in tensor memory
@@ -45,13 +52,25 @@ struct BoundsParams {
     int group_rows, num_groups;       // group g holds the rows [g * group_rows, (g + 1) * group_rows)
     int q_stride;                     // out is [num_groups][q_stride]
     int qt_per_unit, units_q;         // query tiles per work unit, units per tile of rows
-    float keep;
     uint32_t *out;                    // ordered fp32 (float_to_ordered), starts as all ones
     int *failed;                      // set when a bounded wait ran out: the bounds must then not be used
 };
 
-__host__ __device__ inline double bounds_keep(int dim) {
-    return 1.0 - (1.0 / 512 + (double)dim / (1 << 20) + (double)dim / (1 << 23) + 1.0 / (1 << 20));
+constexpr float kLbScale = 1.0f + 0.3214f / 1024;       // s: E[t x] / E[x^2] of truncation errors t for mantissas spread over [1, 2)
+constexpr float kLbRatio = 0.2f / 1024;                 // r
+
+__host__ __device__ inline float bounds_keep(int dim) {
+    return (float)(1.0 - kLbRatio * (1.0 + 1.0 / 256) - (double)dim / (1 << 22) - (double)dim / (1 << 23) - 1.0 / (1 << 20));
+}
+
+// Residual of a coordinate.
+__device__ __forceinline__ float bounds_residual(float x) {
+    return __fmaf_rn(-kLbScale, __uint_as_float(__float_as_uint(x) & 0xFFFFE000u), x);
+}
+
+// query_term from |q|^2 and |dq|^2 (computed in double).
+__device__ __forceinline__ double bounds_query_term(double q2, double dq2, int dim) {
+    return (double)bounds_keep(dim) * q2 - dq2 * (1.001 / kLbRatio);
 }
 
 template <bool PLAIN>
@@ -163,7 +182,7 @@ distance_bounds_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
         for (int u = blockIdx.x; u < units && ok; u += gridDim.x, ++un) {
             const int rt = u / prm.units_q, qt0 = (u % prm.units_q) * prm.qt_per_unit;
             const int qt1 = min(qt0 + prm.qt_per_unit, q_tiles);
-            float nx = 0.0f;
+            float nx = 0.0f, dx = 0.0f;          // |x|^2, |dx|^2
             for (int qt = qt0; qt < qt1 && ok; ++qt) {
                 for (int c = 0; c < nchunks; ++c, ++s_no) {
                     const int st = (int)(s_no % kLbStages);
@@ -196,6 +215,10 @@ distance_bounds_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
                             const float4 v = *reinterpret_cast<const float4 *>(bs + row * 128 + ((j ^ (row & 7)) << 4));
                             nx = __fmaf_rn(v.x, v.x, nx); nx = __fmaf_rn(v.y, v.y, nx);
                             nx = __fmaf_rn(v.z, v.z, nx); nx = __fmaf_rn(v.w, v.w, nx);
+                            const float ex = bounds_residual(v.x), ey = bounds_residual(v.y);
+                            const float ez = bounds_residual(v.z), ew = bounds_residual(v.w);
+                            dx = __fmaf_rn(ex, ex, dx); dx = __fmaf_rn(ey, ey, dx);
+                            dx = __fmaf_rn(ez, ez, dx); dx = __fmaf_rn(ew, ew, dx);
                         }
                     }
                     if (PLAIN) {
@@ -211,7 +234,8 @@ distance_bounds_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
                     if (!ok) break;
                     const bool live = (uint32_t)rt * kLbRows + (uint32_t)row < (uint32_t)prm.n;
                     s_norm[nb][row] = !live ? __int_as_float(0x7F800000)
-                                            : (nx <= kLbMaxNorm ? prm.keep * nx : __int_as_float(0xFF800000));
+                                            : (nx <= kLbMaxNorm ? __fmaf_rn(dx, -1.001f / kLbRatio, bounds_keep(prm.dim) * nx)
+                                                               : __int_as_float(0xFF800000));
                     mbar_arrive(smem_u32(&norm_full[nb]));
                 }
             }
@@ -252,10 +276,10 @@ distance_bounds_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
                         const float4 v = nv[j];
-                        m0 = fminf(m0, fminf(__fmaf_rn(-2.0f, __uint_as_float(r[4 * j]), v.x),
-                                             __fmaf_rn(-2.0f, __uint_as_float(r[4 * j + 1]), v.y)));
-                        m1 = fminf(m1, fminf(__fmaf_rn(-2.0f, __uint_as_float(r[4 * j + 2]), v.z),
-                                             __fmaf_rn(-2.0f, __uint_as_float(r[4 * j + 3]), v.w)));
+                        m0 = fminf(m0, fminf(__fmaf_rn(-2.0f * kLbScale * kLbScale, __uint_as_float(r[4 * j]), v.x),
+                                             __fmaf_rn(-2.0f * kLbScale * kLbScale, __uint_as_float(r[4 * j + 1]), v.y)));
+                        m1 = fminf(m1, fminf(__fmaf_rn(-2.0f * kLbScale * kLbScale, __uint_as_float(r[4 * j + 2]), v.z),
+                                             __fmaf_rn(-2.0f * kLbScale * kLbScale, __uint_as_float(r[4 * j + 3]), v.w)));
                     }
                     const float m = fminf(m0, m1);
                     run = fminf(run, m);

@@ -7,6 +7,7 @@
 //                         k-th distance, and then only the groups whose bound does not exceed it.
 #pragma once
 #include "common.cuh"
+#include "distance_bounds.cuh"
 #include "traverse.cuh"
 
 namespace dci {
@@ -20,10 +21,9 @@ struct ExactParams {
     int *out_ids;                   // slices == 1: the result itself, [nq][knn] ...
     float *out_dists;
     uint64_t *out_packed;           // ... or packed keys instead, when not null
-    const uint32_t *lb;             // nearest_groups_kernel: [num_groups][nq] bounds, rows per group, bound factor
+    const uint32_t *lb;             // nearest_groups_kernel: [num_groups][nq] bounds, rows per group
     const int *failed;
     int num_groups, group_rows, first;
-    float keep;
 };
 
 __device__ __forceinline__ void write_result(const ExactParams &p, int q, const uint64_t *res) {
@@ -99,24 +99,26 @@ nearest_groups_kernel(const ExactParams p) {
     __shared__ int s_count, s_listed;
     __shared__ uint64_t s_thresh;
     __shared__ int s_group[kNgList + kNgThreads];
-    __shared__ double s_sum[kNgThreads / 32];
+    __shared__ double s_sum[2][kNgThreads / 32];
     const int q = blockIdx.x, tid = threadIdx.x;
     uint64_t *bufs = reinterpret_cast<uint64_t *>(dyn_smem);
     float *qv = reinterpret_cast<float *>(dyn_smem + (size_t)p.topk_cap * 16);
-    double s = 0.0;
+    double s = 0.0, t = 0.0;
     for (int c = tid; c < p.dim; c += blockDim.x) {
         const float v = p.query[(size_t)q * p.dim + c];
+        const float e = bounds_residual(v);
         qv[c] = v;
         s += (double)v * v;
+        t += (double)e * e;
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-    if ((tid & 31) == 0) s_sum[tid >> 5] = s;
+    for (int o = 16; o > 0; o >>= 1) { s += __shfl_xor_sync(0xFFFFFFFFu, s, o); t += __shfl_xor_sync(0xFFFFFFFFu, t, o); }
+    if ((tid & 31) == 0) { s_sum[0][tid >> 5] = s; s_sum[1][tid >> 5] = t; }
     if (tid == 0) s_listed = 0;
     CtaTopK topk;
     topk.init(bufs, &s_count, &s_thresh, s_sel, s_res, p.topk_cap, p.knn);      // ends with a barrier
-    double q2 = 0.0;
-    for (int w = 0; w < kNgThreads / 32; ++w) q2 += s_sum[w];
+    double q2 = 0.0, dq2 = 0.0;
+    for (int w = 0; w < kNgThreads / 32; ++w) { q2 += s_sum[0][w]; dq2 += s_sum[1][w]; }
 
     const uint32_t *lb = p.lb + q;
     const size_t stride = (size_t)p.nq;
@@ -141,7 +143,7 @@ nearest_groups_kernel(const ExactParams p) {
             const uint64_t th = s_thresh;
             const float d = __uint_as_float((uint32_t)(th >> 32));
             if (th != kEmptySlot && d < __int_as_float(0x7F800000) && q2 <= 1.0e30)     // as in select_work_kernel
-                limit = __double2float_ru((double)d * d * (1.0 + (p.dim + 8.0) / 8388608.0) + 1.0e-18 - (double)p.keep * q2);
+                limit = __double2float_ru((double)d * d * (1.0 + (p.dim + 8.0) / 8388608.0) + 1.0e-18 - bounds_query_term(q2, dq2, p.dim));
             __syncthreads();
         }
         for (int g0 = 0; g0 < p.num_groups; g0 += blockDim.x) {

@@ -13,6 +13,7 @@
 // 15 partitions first 145, 71, 60 and 73 ms; the rounds of a quarter each make that choice matter less.
 #pragma once
 #include "common.cuh"
+#include "distance_bounds.cuh"
 
 namespace dci {
 
@@ -29,7 +30,6 @@ struct SelectParams {
     int first, step;              // partitions of round 1, and at most of each later round but the last
     int round, last;              // 1, 2, ..; last: 1 in the last round
     int per_item;                 // queries of a partition that a traversal CTA takes together: offs counts such items
-    float keep;
 };
 
 // Starting values of everything the rounds use, in one launch: empty lists, no bound yet, bounds and counters.
@@ -48,7 +48,7 @@ template <bool FIRST>
 __global__ void __launch_bounds__(128) select_work_kernel(const SelectParams p) {
     __shared__ uint32_t s_sel[2][256];
     __shared__ uint32_t s_res[4];
-    __shared__ double s_sum[4];
+    __shared__ double s_sum[2][4];
     __shared__ int s_last;
     __shared__ uint32_t s_scratch[40];
     const int q = blockIdx.x, tid = threadIdx.x;
@@ -80,19 +80,23 @@ __global__ void __launch_bounds__(128) select_work_kernel(const SelectParams p) 
                 cta_select2([lists](int j) { return (uint32_t)(lists[j] >> 32); }, total, p.knn, p.knn, 32, s_sel, s_res, out);
                 kth = out[0];
             }
-            double s = 0.0;           // |q|^2
-            for (int c = tid; c < p.dim; c += blockDim.x) { const double v = p.query[(size_t)q * p.dim + c]; s += v * v; }
+            double s = 0.0, t = 0.0;  // |q|^2 and |dq|^2
+            for (int c = tid; c < p.dim; c += blockDim.x) {
+                const float v = p.query[(size_t)q * p.dim + c], e = bounds_residual(v);
+                s += (double)v * v;
+                t += (double)e * e;
+            }
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-            if ((tid & 31) == 0) s_sum[tid >> 5] = s;
+            for (int o = 16; o > 0; o >>= 1) { s += __shfl_xor_sync(0xFFFFFFFFu, s, o); t += __shfl_xor_sync(0xFFFFFFFFu, t, o); }
+            if ((tid & 31) == 0) { s_sum[0][tid >> 5] = s; s_sum[1][tid >> 5] = t; }
             __syncthreads();
-            const double q2 = (s_sum[0] + s_sum[1]) + (s_sum[2] + s_sum[3]);
+            const double q2 = (s_sum[0][0] + s_sum[0][1]) + (s_sum[0][2] + s_sum[0][3]);
+            const double dq2 = (s_sum[1][0] + s_sum[1][1]) + (s_sum[1][2] + s_sum[1][3]);
             const float d = __uint_as_float(kth);              // an empty slot reads as NaN
             if (d < __int_as_float(0x7F800000) && q2 <= 1.0e30) {
                 // a row is strictly beyond d when its squared distance exceeds d^2 by more than the rounding of
                 // the distance chain (about (dim + 4) 2^-24, twice that taken); 1e-18 covers underflow
-                const double t = (double)d * d * (1.0 + (p.dim + 8.0) / 8388608.0) + 1.0e-18 - (double)p.keep * q2;
-                limit = __double2float_ru(t);
+                limit = __double2float_ru((double)d * d * (1.0 + (p.dim + 8.0) / 8388608.0) + 1.0e-18 - bounds_query_term(q2, dq2, p.dim));
                 if (tid == 0) atomicMin(p.qbound + q, kth);
             }
         }
