@@ -842,13 +842,16 @@ int dci_b200_append(dci_b200_t *h, const float *d_all_data, int num_points_total
             return invalidate(fail(DCI_B200_ERR_CUDA, "%s failed at %s:%d: %s", #call, __FILE__,    \
                                    __LINE__, cudaGetErrorString(e_)));                              \
     } while (0)
-    DCI_CUDA_OR_EMPTY(cudaStreamSynchronize(st));       // growing a buffer frees it: nothing may still read it
+    if (h->keysT.cap < (size_t)I * n_new * sizeof(float))
+        DCI_CUDA_OR_EMPTY(cudaStreamSynchronize(st));   // growing a buffer frees it: nothing may still read it
     DCI_CUDA_OR_EMPTY(h->keysT.ensure((size_t)I * n_new * sizeof(float)));
     if (int rc = launch_project(h, d_all_data + (size_t)n_old * h->dim, n_add, (float *)h->keysT.p, st)) return invalidate(rc);
     DCI_CUDA_OR_EMPTY(cudaMemcpy2DAsync((float *)h->tmp_keys.p + n_old, (size_t)n_new * sizeof(float), h->keysT.p,
                                         (size_t)n_add * sizeof(float), (size_t)n_add * sizeof(float), (size_t)I,
                                         cudaMemcpyDeviceToDevice, st));
-    DCI_CUDA_OR_EMPTY(cudaStreamSynchronize(st));
+    const size_t entry_bytes = (size_t)I * n_new * sizeof(float);
+    if (h->keys.cap < entry_bytes || h->ids.cap < entry_bytes || h->pos.cap < pos_bytes(I, num_parts, ppb, h->T))
+        DCI_CUDA_OR_EMPTY(cudaStreamSynchronize(st));
 #undef DCI_CUDA_OR_EMPTY
     // 3. every segment again, for the partition bounds of the new point count
     if (int rc = ensure_index_buffers(h, (size_t)I * n_new, ppb, num_parts, h->T)) { h->num_points = 0; h->d_data = nullptr; return rc; }
