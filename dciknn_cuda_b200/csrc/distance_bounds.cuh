@@ -38,12 +38,13 @@ namespace dci {
 constexpr int kLbQueries = 128;       // M of the MMA tile
 constexpr int kLbRows = 256;          // N of the MMA tile
 constexpr int kLbK = 32;              // coordinates per stage
-constexpr int kLbStages = 4;
 constexpr int kLbThreads = 512;
 constexpr int kLbNormWarps = 8;
 constexpr size_t kLbABytes = (size_t)kLbQueries * 128, kLbBBytes = (size_t)kLbRows * 128;
-constexpr size_t kLbStageBytes = kLbABytes + kLbBBytes;
-constexpr size_t kLbSmem = kLbStages * kLbStageBytes + 1024;
+// MT query tiles share a tile of rows: 48 KB x 4 stages for one, 64 KB x 3 for two
+__host__ __device__ constexpr int lb_stages(int mt) { return mt == 1 ? 4 : 3; }
+__host__ __device__ constexpr size_t lb_stage_bytes(int mt) { return mt * kLbABytes + kLbBBytes; }
+__host__ __device__ constexpr size_t lb_smem(int mt) { return lb_stages(mt) * lb_stage_bytes(mt) + 1024; }
 constexpr float kLbMaxNorm = 1.0e30f;
 
 struct BoundsParams {
@@ -51,7 +52,7 @@ struct BoundsParams {
     int n, dim, nq;                   // rows, coordinates, queries (of this launch)
     int group_rows, num_groups;       // group g holds the rows [g * group_rows, (g + 1) * group_rows)
     int q_stride;                     // out is [num_groups][q_stride]
-    int qt_per_unit, units_q;         // query tiles per work unit, units per tile of rows
+    int qt_per_unit, units_q;         // query tiles per work unit (a multiple of MT, or all), units per tile of rows
     uint32_t *out;                    // ordered fp32 (float_to_ordered), starts as all ones
     int *failed;                      // set when a bounded wait ran out: the bounds must then not be used
 };
@@ -73,11 +74,17 @@ __device__ __forceinline__ double bounds_query_term(double q2, double dq2, int d
     return (double)bounds_keep(dim) * q2 - dq2 * (1.001 / kLbRatio);
 }
 
-template <bool PLAIN>
+// MT = 2: two query tiles against every staged tile of rows, an accumulator each (so none to spare for the next tile,
+// whose products wait for the minima of this one).  A third fewer bytes per product through L2, which is what bounds
+// one tile (91 bytes per SM and cycle at the full tensor rate); it pays where rows are long, see launch_bounds.
+template <bool PLAIN, int MT>
 __global__ void __launch_bounds__(kLbThreads, 1)
 distance_bounds_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_q,
                        const BoundsParams prm) {
-    extern __shared__ __align__(16) unsigned char lb_smem[];
+    static_assert(!PLAIN || MT == 1, "ordinary loads stage one query tile");
+    constexpr int kLbStages = lb_stages(MT);
+    constexpr size_t kLbStageBytes = lb_stage_bytes(MT);
+    extern __shared__ __align__(16) unsigned char lb_dyn[];
     __shared__ __align__(8) unsigned long long full_bar[kLbStages], empty_bar[kLbStages];
     __shared__ __align__(8) unsigned long long acc_full[2], acc_empty[2], norm_full[2], norm_empty[2];
     __shared__ __align__(16) float s_norm[2][kLbRows];
@@ -85,8 +92,8 @@ distance_bounds_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
     __shared__ volatile int abort_flag;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t s0 = smem_u32(lb_smem);
-    unsigned char *base = lb_smem + (((s0 + 1023u) & ~1023u) - s0);
+    const uint32_t s0 = smem_u32(lb_dyn);
+    unsigned char *base = lb_dyn + (((s0 + 1023u) & ~1023u) - s0);
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
@@ -126,7 +133,7 @@ distance_bounds_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
         for (int u = blockIdx.x; u < units && !abort_flag; u += gridDim.x) {
             const int rt = u / prm.units_q, qt0 = (u % prm.units_q) * prm.qt_per_unit;
             const int qt1 = min(qt0 + prm.qt_per_unit, q_tiles);
-            for (int qt = qt0; qt < qt1 && !abort_flag; ++qt)
+            for (int qt = qt0; qt < qt1 && !abort_flag; qt += MT)
                 for (int c = 0; c < nchunks; ++c, ++s_no) {
                     const int st = (int)(s_no % kLbStages);
                     const uint32_t use = s_no / kLbStages;
@@ -134,13 +141,15 @@ distance_bounds_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
                     const uint32_t a = smem_u32(base + (size_t)st * kLbStageBytes), bar = smem_u32(&full_bar[st]);
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)kLbStageBytes)
                                  : "memory");
+#pragma unroll
+                    for (int m = 0; m < MT; ++m)             // (a tile beyond the queries reads as zeros)
+                        asm volatile(
+                            "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::
+                                "r"(a + (uint32_t)(m * kLbABytes)), "l"(&map_q), "r"(c * kLbK), "r"((qt + m) * kLbQueries), "r"(bar)
+                            : "memory");
                     asm volatile(
                         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::
-                            "r"(a), "l"(&map_q), "r"(c * kLbK), "r"(qt * kLbQueries), "r"(bar)
-                        : "memory");
-                    asm volatile(
-                        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::
-                            "r"(a + (uint32_t)kLbABytes), "l"(&map_x), "r"(c * kLbK), "r"(rt * kLbRows), "r"(bar)
+                            "r"(a + (uint32_t)(MT * kLbABytes)), "l"(&map_x), "r"(c * kLbK), "r"(rt * kLbRows), "r"(bar)
                         : "memory");
                 }
         }
@@ -154,24 +163,32 @@ distance_bounds_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
         uint32_t s_no = 0, t = 0;
         for (int u = blockIdx.x; u < units && !abort_flag; u += gridDim.x) {
             const int qt0 = (u % prm.units_q) * prm.qt_per_unit, qt1 = min(qt0 + prm.qt_per_unit, q_tiles);
-            for (int qt = qt0; qt < qt1 && !abort_flag; ++qt, ++t) {
-                const int a = (int)(t & 1u);
-                if (t > 1 && !mbar_wait(smem_u32(&acc_empty[a]), ((t >> 1) - 1) & 1u)) { abort_flag = 1; break; }
+            for (int qt = qt0; qt < qt1 && !abort_flag; qt += MT, ++t) {
+                const int a = MT == 1 ? (int)(t & 1u) : 0;
+                const uint32_t earlier = MT == 1 ? t >> 1 : t;       // tiles that used this accumulator before
+                if (earlier > 0)
+                    for (int m = 0; m < MT; ++m)
+                        if (!mbar_wait(smem_u32(&acc_empty[a + m]), (earlier - 1) & 1u)) { abort_flag = 1; break; }
+                if (abort_flag) break;
                 const uint32_t tmem_d = tmem_base + (uint32_t)(a * kLbRows);
                 for (int c = 0; c < nchunks; ++c, ++s_no) {
                     const int st = (int)(s_no % kLbStages);
                     if (!mbar_wait(smem_u32(&full_bar[st]), (s_no / kLbStages) & 1u)) { abort_flag = 1; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t as = smem_u32(base + (size_t)st * kLbStageBytes), bs = as + (uint32_t)kLbABytes;
+                    const uint32_t as = smem_u32(base + (size_t)st * kLbStageBytes), bs = as + (uint32_t)(MT * kLbABytes);
 #pragma unroll
                     for (int kk = 0; kk < kLbK / 8; ++kk)
-                        umma_tf32(tmem_d, umma_desc_sw128(as + kk * 32), umma_desc_sw128(bs + kk * 32), idesc, (c | kk) ? 1u : 0u);
+#pragma unroll
+                        for (int m = 0; m < MT; ++m)
+                            umma_tf32(tmem_d + m * kLbRows, umma_desc_sw128(as + (uint32_t)(m * kLbABytes) + kk * 32),
+                                      umma_desc_sw128(bs + kk * 32), idesc, (c | kk) ? 1u : 0u);
                     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                                      smem_u32(&empty_bar[st])) : "memory");
                 }
                 if (abort_flag) break;
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                                 smem_u32(&acc_full[a])) : "memory");
+                for (int m = 0; m < MT; ++m)
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                                     smem_u32(&acc_full[a + m])) : "memory");
             }
         }
     } else if (warp >= 8) {
@@ -183,11 +200,11 @@ distance_bounds_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
             const int rt = u / prm.units_q, qt0 = (u % prm.units_q) * prm.qt_per_unit;
             const int qt1 = min(qt0 + prm.qt_per_unit, q_tiles);
             float nx = 0.0f, dx = 0.0f;          // |x|^2, |dx|^2
-            for (int qt = qt0; qt < qt1 && ok; ++qt) {
+            for (int qt = qt0; qt < qt1 && ok; qt += MT) {
                 for (int c = 0; c < nchunks; ++c, ++s_no) {
                     const int st = (int)(s_no % kLbStages);
                     const uint32_t use = s_no / kLbStages;
-                    unsigned char *as = base + (size_t)st * kLbStageBytes, *bs = as + kLbABytes;
+                    unsigned char *as = base + (size_t)st * kLbStageBytes, *bs = as + MT * kLbABytes;
                     if (PLAIN) {
                         ok = warp_ok(use == 0 || mbar_wait(smem_u32(&empty_bar[st]), (use - 1) & 1u));
                         if (!ok) break;
@@ -254,7 +271,9 @@ distance_bounds_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
             const int r0 = rt * kLbRows;
             const int g_first = r0 / prm.group_rows;
             const int end_first = (int)min((long long)(g_first + 1) * prm.group_rows - r0, (long long)prm.n);   // column at which that group ends
-            for (int qt = qt0; qt < qt1; ++qt, ++t) {
+            // one accumulator after the other; with MT = 2 a unit that ends on an odd tile still has both (zeros)
+            const int tiles = (qt1 - qt0 + MT - 1) / MT * MT;
+            for (int qt = qt0; qt < qt0 + tiles; ++qt, ++t) {
                 const int a = (int)(t & 1u);
                 ok = warp_ok(mbar_wait(smem_u32(&acc_full[a]), (t >> 1) & 1u));
                 if (!ok) break;

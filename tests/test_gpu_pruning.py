@@ -31,7 +31,9 @@ SIZES = [(2048, 32, 128, 8, 2, 4, 10, 10, 100, "latent"),      # everything a mu
          (8193, 8, 1185, 10, 1, 2, 16, 1, 900, "mixture"),     # more queries than fit the scan
          (8192, 64, 129, 7, 2, 3, 7, 128, 1280, "unit"),
          (4097, 12, 40, 5, 2, 3, 10, 300, 3000, "latent"),
-         (6000, 960, 9, 4, 1, 3, 10, 10, 10000, "unit")]
+         (6000, 960, 9, 4, 1, 3, 10, 10, 10000, "unit"),
+         (3000, 516, 300, 6, 1, 3, 10, 5, 50, "latent"),       # long rows, an odd number of query tiles taken two at a time
+         (3000, 512, 256, 4, 1, 3, 10, 5, 1000, "latent")]
 
 
 def _rows(rng, n, dim, dist):
