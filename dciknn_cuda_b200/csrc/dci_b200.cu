@@ -345,13 +345,13 @@ int pick_buckets(dci_b200 *h, dci::TraverseParams &prm, int nthreads, size_t sta
     return std::min(std::max(prm.wcap / 2, 64), 16384);
 }
 
-// CTAs of the traversal kernels per SM: shared memory, threads, and 64 registers a thread.
-int traverse_ctas_per_sm(const dci_b200 *h, size_t smem, int nthreads) {
-    return (int)std::max<size_t>(1, std::min<size_t>(h->smem_per_sm / (smem + 1024), 1024 / nthreads));
-}
+// CTAs of the traversal kernels that an SM holds at a time: 64 registers a thread beside the grid's own limits.  The
+// grid itself is not cut to that: the CTAs beyond it start as others end, which evens their work out (650k x 96 in 400
+// partitions, 7 queries: 549 us a cycle, 565 with a grid of what is resident).
+int traverse_resident_per_sm(int per_sm, int nthreads) { return std::min(per_sm, std::max(1, 1024 / nthreads)); }
 
 // How a traversal runs: work arrays in shared memory or in a slab of device memory per CTA, CTAs per SM.
-struct TraverseGeometry { bool smem; size_t dyn, per_cta; int per_sm; };
+struct TraverseGeometry { bool smem; size_t dyn, per_cta; int per_sm, resident; };
 
 // Works the geometry out and sets what depends on it in prm (buckets, query groups, slab layout).
 template <typename ValT, typename PosT>
@@ -386,8 +386,8 @@ int plan_traverse(dci_b200 *h, dci::TraverseParams &prm, int nthreads, TraverseG
     }
     prm.topk_global_off = lay.fallback_bytes + (smem ? 0 : lay.big_bytes);
     const size_t per_cta = prm.topk_global_off + (prm.topk_global ? (size_t)prm.topk_cap * 16 : 0);
-    const int per_sm = traverse_ctas_per_sm(h, dyn + static_smem, nthreads);
-    *geo = {smem, dyn, per_cta, per_sm};
+    const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(h->smem_per_sm / (dyn + static_smem + 1024), 2048 / nthreads));
+    *geo = {smem, dyn, per_cta, per_sm, traverse_resident_per_sm(per_sm, nthreads)};
     return 0;
 }
 
@@ -1061,7 +1061,7 @@ static int query_impl(dci_b200_t *h, const float *d_query, int num_queries, int 
                                          : (p.wcap <= 65535 ? plan_traverse<uint16_t, uint16_t>(h, p, nthreads, &geo)
                                                             : plan_traverse<uint32_t, uint16_t>(h, p, nthreads, &geo));
                 if (!rc)
-                    rc = traverse_pruned(h, prm, prune_first, p.qbatch, (long long)h->sm_count * geo.per_sm, (unsigned char *)h->prune.p,
+                    rc = traverse_pruned(h, prm, prune_first, p.qbatch, (long long)h->sm_count * geo.resident, (unsigned char *)h->prune.p,
                                          st, traverse);
             } else {
                 rc = traverse(prm);
@@ -1612,13 +1612,9 @@ int query_noalloc_impl(dci_b200 *h, dci::TraverseParams prm, int nthreads, unsig
     if (!smem) lay = dci::TraverseLayout<ValT>::make(nthreads, prm.dim, prm.topk_cap, prm.L, prm.wcap, prm.ppb, prm.nbuckets, false, prm.bkey != 0);
     const size_t dyn = smem ? lay.fixed_bytes + lay.big_bytes : lay.fixed_bytes;
     const size_t per_cta = align256(lay.fallback_bytes + (smem ? 0 : lay.big_bytes));
-    // the slabs set aside (and with them what is refused) count CTAs without regard to registers; the grid is what an
-    // SM really holds
-    const int slabs_per_sm = (int)std::max<size_t>(1, std::min<size_t>(h->smem_per_sm / (dyn + static_smem + 1024), 2048 / nthreads));
-    const int per_sm = std::min(slabs_per_sm, traverse_ctas_per_sm(h, dyn + static_smem, nthreads));
-    const long long slab_count = std::min<long long>((long long)num_queries * prm.num_parts, (long long)h->sm_count * slabs_per_sm);
+    const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(h->smem_per_sm / (dyn + static_smem + 1024), 2048 / nthreads));
     const long long max_grid = std::min<long long>((long long)num_queries * prm.num_parts, (long long)h->sm_count * per_sm);
-    const size_t slabs = per_cta * (size_t)slab_count;
+    const size_t slabs = per_cta * (size_t)max_grid;
     // per query of a pass: its per-partition result lists and its word of the shared distance bound
     const size_t per_query = sizeof(uint64_t) * (size_t)prm.num_parts * prm.kpart + sizeof(uint32_t);
     int prune_first = prune_first_round(h, prm, num_queries);
@@ -1663,7 +1659,7 @@ int query_noalloc_impl(dci_b200 *h, dci::TraverseParams prm, int nthreads, unsig
             DCI_CUDA(cudaGetLastError());
             return 0;
         };
-        if (int rc = prune_first ? traverse_pruned(h, prm, prune_first, 1, (long long)h->sm_count * per_sm, scratch + lists_end, st, traverse) : traverse(prm)) return rc;
+        if (int rc = prune_first ? traverse_pruned(h, prm, prune_first, 1, (long long)h->sm_count * traverse_resident_per_sm(per_sm, nthreads), scratch + lists_end, st, traverse) : traverse(prm)) return rc;
         dci::merge_partitions_kernel<<<prm.nq, merge_threads, (size_t)merge_cap * 16, st>>>(
             prm.part_topk, prm.num_parts, prm.kpart, prm.knn, merge_cap, q0, prm.nq, nullptr, d_ids, d_dists, 0);
         h->launches++;
