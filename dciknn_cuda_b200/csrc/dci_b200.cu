@@ -615,7 +615,7 @@ ExactPlan plan_exact(const dci_b200 *h, const dci::TraverseParams &prm, int num_
     const size_t per_query = sizeof(uint32_t) * (size_t)g.num_groups;
     g.batch = (int)std::min<size_t>((size_t)num_queries, (std::min<size_t>(avail, (size_t)256 << 20) - 512) / per_query);
     g.bytes = per_query * g.batch + 512;
-    if (g.num_groups < 2 * g.first || g.batch < 1 || (g.batch < num_queries && g.batch < 1024)) return p;
+    if (g.num_groups < 2 * g.first || g.batch < 1 || g.bytes > avail || (g.batch < num_queries && g.batch < 1024)) return p;
     if (h->pruning == 1) return g;
     if (g.num_groups < 4 * g.first) return p;
     const double scan_us = 8.0 + cells * num_queries * 4.0 / 5.0e6;
