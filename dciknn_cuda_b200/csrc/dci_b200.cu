@@ -854,9 +854,10 @@ int dci_b200_append(dci_b200_t *h, const float *d_all_data, int num_points_total
     DCI_CUDA_OR_EMPTY(cudaMemcpy2DAsync((float *)h->tmp_keys.p + n_old, (size_t)n_new * sizeof(float), h->keysT.p,
                                         (size_t)n_add * sizeof(float), (size_t)n_add * sizeof(float), (size_t)I,
                                         cudaMemcpyDeviceToDevice, st));
-    const size_t entry_bytes = (size_t)I * n_new * sizeof(float);
-    if (h->keys.cap < entry_bytes || h->ids.cap < entry_bytes || h->pos.cap < pos_bytes(I, num_parts, ppb, h->T))
-        DCI_CUDA_OR_EMPTY(cudaStreamSynchronize(st));
+    // The call's promise: when it returns, everything queued on the stream before it and its own reads of the rows are
+    // over, so the caller may release the rows that d_all_data replaces, whatever stream they came from (DCI.append drops
+    // them).  The buffers that grow below need it too.
+    DCI_CUDA_OR_EMPTY(cudaStreamSynchronize(st));
 #undef DCI_CUDA_OR_EMPTY
     // 3. every segment again, for the partition bounds of the new point count
     if (int rc = ensure_index_buffers(h, (size_t)I * n_new, ppb, num_parts, h->T)) { h->num_points = 0; h->d_data = nullptr; return rc; }

@@ -97,7 +97,10 @@ int dci_b200_add(dci_b200_t *h, const float *d_data, int num_points, int block_s
  * segment is then sorted again for the partition bounds of the new count
  * (ppb = ceil(num_points_total / P), with the P and T of the first add).  The
  * result is the index dci_b200_add would build from d_all_data, bit for bit.
- * The index borrows d_all_data from then on.  Synchronises the stream. */
+ * The index borrows d_all_data from then on.  Synchronises the stream after the
+ * last access to the rows: when the call returns, work queued on it earlier (the
+ * copy into d_all_data) and the projection are over, and the array that
+ * d_all_data replaces may be released; the sorting may still be pending. */
 int dci_b200_append(dci_b200_t *h, const float *d_all_data, int num_points_total, void *stream);
 
 /* Replaces dci_query (include/dci.h:71-75, src/dci_cuda_kernel.cu:777-875) and

@@ -65,3 +65,37 @@ def test_append_argument_and_state_errors():
     d.add(x)                                      # usable again after clear
     assert d.num_points == 100
     d.free()
+
+
+def test_append_waits_for_the_rows_it_replaces():
+    """append drops the old rows, so it must not return while its stream still has to copy them -- also when no buffer
+    grows (the second clear / add / append cycle), and when the rows came from another stream's memory pool."""
+    rng = np.random.default_rng(5)
+    n, e, dim = 20000, 500, 32
+    rows = rng.standard_normal((n + e, dim)).astype(np.float32)
+    proj = cases.unit_rows(rng, 10, dim)
+    more = torch.from_numpy(rows[n:]).cuda()
+    d = DCI(dim, 2, 5, 10, 10, proj=torch.from_numpy(proj))
+    side = torch.cuda.Stream()
+    for cycle in range(3):
+        d.clear()
+        kept = torch.from_numpy(rows[:n]).cuda() if cycle < 2 else None      # the last cycle leaves the rows to the index
+        d.add(torch.from_numpy(rows[:n]).cuda() if kept is None else kept)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(20_000_000)          # about 10 ms of a busy stream before the copy of the old rows
+            queued = torch.cuda.Event()
+            queued.record()
+            d.append(more)
+            assert queued.query(), "append returned before the work queued ahead of it was done"
+        garbage = [torch.full((n, dim), 1e9, device="cuda") for _ in range(3)]      # takes memory that the old rows gave back
+        side.synchronize()
+        del garbage
+    f = _fresh(dim, 2, 5, 10, 10, proj, rows)
+    for a, b in zip(d.get_index(), f.get_index()):
+        assert np.array_equal(np.asarray(a).view(np.uint32), np.asarray(b).view(np.uint32))
+    q = torch.from_numpy(rows[:40] + np.float32(0.1)).cuda()
+    for a, b in zip(d.query(q, 10, return_int_ids=True), f.query(q, 10, return_int_ids=True)):
+        assert torch.equal(a.cpu(), b.cpu())
+    d.free()
+    f.free()
