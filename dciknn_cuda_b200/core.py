@@ -404,6 +404,13 @@ class DCI(object):
         it pay; 1: wherever possible; 2: never.  Results do not depend on it."""
         _capi.check(_capi.lib().dci_b200_set_pruning(self._live(), int(mode)))
 
+    def last_call(self):
+        """Which way the last call went (a diagnostic): the kernel of the last projection, 'staged' (rows staged by
+        the computing threads), 'tma' or 'small' (few points)."""
+        buf = (C.c_longlong * 8)()
+        _capi.check(_capi.lib().dci_b200_last_call(self._live(), buf))
+        return dict(projection=("staged", "tma", "small")[buf[0]])
+
     def set_max_ctas(self, max_ctas):
         """Caps the number of CTAs of the traversal kernel (0 = automatic).  For tests: with few CTAs
         every CTA works through many (query, partition) pairs one after the other."""

@@ -130,7 +130,7 @@ struct dci_b200 {
     int stats_on = 0, stats_nq = 0, phases_valid = 0;
     int timing_on = 0;
     int last_qbatch = 1;                 // queries per CTA pass of the last traversal launch
-    int last_projection_tma = 0;
+    int last_projection = 0;             // kernel of the last projection: 0 rows staged by the computing threads, 1 fed by TMA, 2 few points
     int projection_mode = 0;             // 0: exact fp32 FMA order, 1: tensor cores, 3xTF32
     Buf errflag;
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -186,7 +186,7 @@ int launch_project(dci_b200 *h, const float *d_x, long long n, float *d_out, cud
         else if (tma)
             DCI_CUDA(cudaFuncSetAttribute(dci::project_tf32x3_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)dci::kTcTmaSmem));
-        h->last_projection_tma = tma ? 1 : 0;
+        h->last_projection = tma ? 1 : 0;
         timer.start();
         for (int i0 = 0; i0 < I; i0 += dci::kTcDirs) {
             if (persistent)
@@ -209,12 +209,21 @@ int launch_project(dci_b200 *h, const float *d_x, long long n, float *d_out, cud
         if (flag) return fail(DCI_B200_ERR_CUDA, "tensor-core projection: a wait on the MMA barrier timed out");
         return 0;
     }
-    // Few points (a query batch, a small set): tiles of 32 points.  Its time grows with points x directions x
-    // coordinates (about 1 us per 10^7 beside 4 us); the TMA-fed kernel needs 14 us for its first tiles.
-    if (h->exact_tma && I <= dci::kPsmMaxIndices && (double)n * I * h->dim <= 1.0e8) {
+    // Few points (a query batch, a small set): tiles of 32 points.  A tile costs the same however few coordinates or
+    // directions it has (64 coordinates are copied at a time, by at least 128 threads), so the line lies at a number of
+    // points x directions (16 at least), and higher where the kernel that it stands in for is the slower one: the TMA-fed
+    // one with more than 12 accumulators a point, the one that stages the rows itself.  us a call, this kernel / the other,
+    // with 10 to 11 us of host side in each:
+    //   TMA-fed, up to 12 directions  10 000 points x 5 directions x 256 coordinates: 13 / 15, 20 000: 17 / 15; 5M x 2 x 8: 431 / 48
+    //   TMA-fed, more                 20 000 x 14 x 256: 21 / 25;  10 000 x 20 x 128: 11 / 15, 20 000: 17 / 15;  300 000 x 20 x 8: 56 / 13
+    //   staging                       20 000 x 20 x 65: 15 / 17, 50 000: 23 / 21;  10 000 x 48 x 128: 19 / 48;  20 000 x 48 x 8: 15 / 11
+    const bool by_tma = I <= 40 && n >= 1024 && h->dim % 4 == 0 && ((uintptr_t)d_x & 15) == 0;
+    const double few = !by_tma ? 5.0e5 : (I <= 12 ? 2.0e5 : 3.2e5);
+    if (h->exact_tma && I <= dci::kPsmMaxIndices && (double)n * std::max(I, 16) <= few &&
+        (double)n * I * h->dim <= 1.0e8) {
         const int threads = std::max(128, (8 * I + 31) & ~31);
         const size_t dyn = 2 * dci::psm_buffer_floats(I) * sizeof(float);      // at most 43 KB
-        h->last_projection_tma = 0;
+        h->last_projection = 2;
         timer.start();
         dci::project_small_kernel<<<(unsigned)((n + dci::kPsmRows - 1) / dci::kPsmRows), threads, dyn, st>>>(d_x, n, h->dim, h->d_proj, I, d_out);
         timer.stop();
@@ -246,7 +255,7 @@ int launch_project(dci_b200 *h, const float *d_x, long long n, float *d_out, cud
                 timer.stop();
                 h->launches++;
                 DCI_CUDA(cudaGetLastError());
-                h->last_projection_tma = 1;
+                h->last_projection = 1;
                 return 0;
             };
             switch (dirs) {
@@ -258,7 +267,7 @@ int launch_project(dci_b200 *h, const float *d_x, long long n, float *d_out, cud
             }
         }
     }
-    h->last_projection_tma = 0;
+    h->last_projection = 0;
     const unsigned grid = (unsigned)((n + dci::kProjPoints - 1) / dci::kProjPoints);
     timer.start();
     // fewest passes over the points, then the smallest accumulator count that achieves it
@@ -1227,7 +1236,15 @@ int dci_b200_get_phase_cycles(dci_b200_t *h, long long *h_out) {
     DCI_CUDA(cudaDeviceSynchronize());
     DCI_CUDA(cudaMemcpy(h_out, h->phases.p, sizeof(long long) * 16, cudaMemcpyDeviceToHost));
     h_out[11] = h->last_qbatch;
-    h_out[13] = h->last_projection_tma;
+    h_out[13] = h->last_projection == 1 ? 1 : 0;
+    return 0;
+}
+
+int dci_b200_last_call(dci_b200_t *h, long long *h_out) {
+    if (int rc = check_handle(h)) return rc;
+    if (!h_out) return fail(DCI_B200_ERR_ARG, "h_out is null");
+    for (int i = 0; i < 8; ++i) h_out[i] = 0;
+    h_out[0] = h->last_projection;
     return 0;
 }
 

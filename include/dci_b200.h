@@ -219,6 +219,11 @@ long long dci_b200_device_alloc_calls(void);
  * row, so tests reach whatever a CTA keeps from one pair to the next. */
 int dci_b200_set_max_ctas(dci_b200_t *h, int max_ctas);
 
+/* Which way the handle's last call went, into 8 words; a diagnostic, for tests.
+ * [0] kernel of the last projection: 0 rows staged by the computing threads,
+ * 1 fed by TMA, 2 the one for few points.  The rest is 0. */
+int dci_b200_last_call(dci_b200_t *h, long long *h_out);
+
 /* Whether queries leave out what provably cannot change their answer: partitions beyond the candidates already
  * known (dciknn_cuda_b200/csrc/prune.cuh), or the whole traversal where every point is a candidate
  * (csrc/exhaustive.cuh).  0, the default, where the sizes of the call make it pay; 1 wherever it is possible;

@@ -73,7 +73,7 @@ def test_directions_unit_norm_and_seeded():
 
 
 @pytest.mark.parametrize("n,dim,L,S", [(1000, 100, 2, 7), (777, 37, 3, 12), (5000, 128, 2, 10), (300, 960, 3, 12), (64, 8, 1, 1),
-                                       # at least 1024 rows of a multiple of 4 coordinates: rows streamed by TMA copies
+                                       # few points whose rows a tensor map could describe; beyond them (70 000) rows streamed by TMA copies
                                        (3001, 100, 2, 6), (1500, 36, 1, 8), (2049, 960, 3, 12), (1025, 8, 1, 1),
                                        (70000, 96, 2, 10), (4100, 256, 2, 15), (4096, 44, 4, 10),
                                        (2000, 130, 2, 5), (3000, 128, 6, 7)])      # dim % 4 != 0, more than 40 directions
@@ -94,6 +94,26 @@ def test_projection_bit_exact(n, dim, L, S):
             pad[1:] = xd.reshape(-1)
             got = g.project(pad[1:].view(n, dim)).cpu().numpy()
             assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("n,dim,L,S,kernel", [
+    # either side of the lines between the kernel for few points and the others: points x directions (16 at least) up to
+    # 2e5 and 3.2e5 where rows can be fed by TMA (12 directions and more), 5e5 where they cannot
+    (12500, 24, 1, 8, "small"), (12501, 24, 1, 8, "tma"), (16000, 32, 2, 10, "small"), (16001, 32, 2, 10, "tma"),
+    (31250, 9, 1, 2, "small"), (31251, 9, 1, 2, "staged"), (10416, 16, 3, 16, "small"), (10417, 16, 3, 16, "staged"),
+    (1023, 8, 3, 16, "small"), (60000, 4, 1, 1, "tma"),
+    # the TMA-fed kernel with every number of accumulators, ragged last tiles, two CTAs on an SM and one
+    (12543, 100, 1, 8, "tma"), (12999, 100, 2, 6, "tma"), (13001, 36, 1, 8, "tma"), (10337, 960, 1, 20, "tma"),
+    (10801, 256, 2, 15, "tma"), (5563, 960, 3, 12, "tma"), (8031, 44, 4, 10, "tma"), (12641, 8, 1, 1, "tma")])
+def test_projection_bit_exact_on_either_side_of_the_line(n, dim, L, S, kernel):
+    from dciknn_cuda_b200 import DCI
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((n, dim)).astype(np.float32)
+    proj = cases.unit_rows(rng, L * S, dim)
+    g = DCI(dim, L, S, proj=torch.from_numpy(proj))
+    got = g.project(torch.from_numpy(x).cuda()).cpu().numpy()
+    assert np.array_equal(got.view(np.uint32), oracle.project(proj, x).view(np.uint32))
+    assert g.last_call()["projection"] == kernel
 
 
 @pytest.mark.parametrize("N,P", [(2000, 100), (103, 10), (13, 40), (10000, 1), (30000, 2), (70000, 1), (140000, 2)])
