@@ -399,17 +399,20 @@ class DCI(object):
             raise RuntimeError(_capi.lib().dci_b200_last_error().decode())
         _capi.check(rc)
 
-    def set_pruning(self, mode):
+    def set_pruning(self, mode, max_bytes=None):
         """0 (default): leave out work that provably cannot change an answer where the sizes of the call make
-        it pay; 1: wherever possible; 2: never.  Results do not depend on it."""
+        it pay; 1: wherever possible; 2: never.  Results do not depend on it.  max_bytes: device memory that the
+        index may hold for it (None: no limit); a call that needs more goes without."""
         _capi.check(_capi.lib().dci_b200_set_pruning(self._live(), int(mode)))
+        _capi.check(_capi.lib().dci_b200_set_pruning_limit(self._live(), -1 if max_bytes is None else int(max_bytes)))
 
     def last_call(self):
         """Which way the last call went (a diagnostic): the kernel of the last projection, 'staged' (rows staged by
-        the computing threads), 'tma' or 'small' (few points)."""
+        the computing threads), 'tma' or 'small' (few points), and the path of the last query: 'all' (query, partition)
+        pairs, 'pruned', or, where every point is a candidate, 'scan' (every row) or 'groups' (of rows, by bounds)."""
         buf = (C.c_longlong * 8)()
         _capi.check(_capi.lib().dci_b200_last_call(self._live(), buf))
-        return dict(projection=("staged", "tma", "small")[buf[0]])
+        return dict(projection=("staged", "tma", "small")[buf[0]], path=("all", "pruned", "scan", "groups")[buf[1]])
 
     def set_max_ctas(self, max_ctas):
         """Caps the number of CTAs of the traversal kernel (0 = automatic).  For tests: with few CTAs

@@ -126,6 +126,8 @@ struct dci_b200 {
     int max_ctas = 0;                    // > 0: cap on the traversal grid (dci_b200_set_max_ctas)
     Buf tmp_keys, qproj, part_topk, scratch, merge_scratch, stats, phases, hq, hids, hdists, qbound, prune;
     int pruning = 0;                     // 0: by the rule of prune_first_round, 1: wherever possible, 2: never
+    size_t pruning_limit = ~(size_t)0;   // bytes that `prune` may take (dci_b200_set_pruning_limit)
+    int last_path = 0;                   // of the last query: 0 every pair traversed, 1 pruned, 2 every row, 3 nearest groups
     int distance_bound = 1;              // 1: share a per-query distance bound between partitions
     int stats_on = 0, stats_nq = 0, phases_valid = 0;
     int timing_on = 0;
@@ -508,6 +510,15 @@ int launch_bounds(dci_b200 *h, const dci::TraverseParams &prm, int group_rows, i
     return two ? go(dci::distance_bounds_kernel<false, 2>, dci::lb_smem(2)) : go(dci::distance_bounds_kernel<false, 1>, dci::lb_smem(1));
 }
 
+// Working memory for leaving work out.  A call answers without it just as well, so no memory (or not that much allowed)
+// is no error: false, and the caller traverses every pair.
+bool pruning_memory(dci_b200 *h, size_t bytes) {
+    if (bytes > h->pruning_limit) return false;
+    if (h->prune.ensure(bytes) == cudaSuccess) return true;
+    cudaGetLastError();      // the failed allocation must not surface at the next launch
+    return false;
+}
+
 // One batch with pruning: bounds, then the rounds.  traverse(prm) launches the traversal of prm's work list.
 // ws: PruneSpace::make(num_parts, nq).bytes of device memory; prm.qbound and prm.part_topk are set.
 // per_item: queries that a traversal CTA takes together; resident: CTAs that run at the same time.
@@ -523,6 +534,7 @@ int traverse_pruned(dci_b200 *h, dci::TraverseParams prm, int first, int per_ite
     // Each costs a last wave of CTAs: 67 waves of 1.25M x 96 and 29 of 100k x 50 lose 2 % with one round more, 675 waves of
     // 1M x 128 go from 71 to 52 ms with two.
     const int rounds = waves < 100.0 ? 2 : (waves < 300.0 ? 3 : 4);
+    h->last_path = 1;
     const PruneSpace sp = PruneSpace::make(prm.num_parts, prm.nq);
     uint32_t *lb = (uint32_t *)(ws + sp.lb);
     int *zero = (int *)(ws + sp.zero);
@@ -637,6 +649,7 @@ ExactPlan plan_exact(const dci_b200 *h, const dci::TraverseParams &prm, int num_
 // ws: plan.bytes of working memory.
 int launch_exact(dci_b200 *h, const ExactPlan &plan, const dci::TraverseParams &prm, const float *d_query, int num_queries,
                  unsigned char *ws, int *d_ids, float *d_dists, unsigned long long *d_packed, cudaStream_t st) {
+    h->last_path = plan.mode == 2 ? 3 : 2;
     for (int q0 = 0; q0 < num_queries; q0 += plan.batch) {
         dci::ExactParams e;
         memset(&e, 0, sizeof(e));
@@ -1006,9 +1019,9 @@ static int query_impl(dci_b200_t *h, const float *d_query, int num_queries, int 
         prm.work_stats = (long long *)h->stats.p;
         h->stats_nq = num_queries;
     }
+    h->last_path = 0;
     const ExactPlan exact = plan_exact(h, prm, num_queries, ~(size_t)0);
-    if (exact.mode) {      // no index entry is looked at: neither projections nor a traversal
-        DCI_CUDA(h->prune.ensure(exact.bytes));
+    if (exact.mode && pruning_memory(h, exact.bytes)) {      // no index entry is looked at: neither projections nor a traversal
         if (timing) { DCI_CUDA(cudaEventRecord(h->ev[2], st)); }
         if (int rc = launch_exact(h, exact, prm, d_query, num_queries, (unsigned char *)h->prune.p, d_ids, d_dists, d_packed, st)) return rc;
         h->last_qbatch = 1;
@@ -1027,8 +1040,8 @@ static int query_impl(dci_b200_t *h, const float *d_query, int num_queries, int 
     const size_t per_query = sizeof(uint64_t) * (size_t)h->num_parts * prm.kpart;
     const int batch = (int)std::max<size_t>(1, std::min<size_t>((size_t)num_queries, ((size_t)1 << 30) / per_query));
     DCI_CUDA(h->part_topk.ensure(per_query * batch + 16));
-    const int prune_first = prune_first_round(h, prm, std::min(batch, num_queries));
-    if (prune_first) DCI_CUDA(h->prune.ensure(PruneSpace::make(h->num_parts, batch).bytes));
+    int prune_first = prune_first_round(h, prm, std::min(batch, num_queries));
+    if (prune_first && !pruning_memory(h, PruneSpace::make(h->num_parts, batch).bytes)) prune_first = 0;
     prm.part_topk = (uint64_t *)h->part_topk.p;
     const int merge_grid_cap = merge_global ? 2 * h->sm_count : (1 << 30);
     if (merge_global) DCI_CUDA(h->merge_scratch.ensure((size_t)merge_grid_cap * 2 * merge_cap * sizeof(uint64_t)));
@@ -1245,6 +1258,7 @@ int dci_b200_last_call(dci_b200_t *h, long long *h_out) {
     if (!h_out) return fail(DCI_B200_ERR_ARG, "h_out is null");
     for (int i = 0; i < 8; ++i) h_out[i] = 0;
     h_out[0] = h->last_projection;
+    h_out[1] = h->last_path;
     return 0;
 }
 
@@ -1263,6 +1277,17 @@ int dci_b200_set_pruning(dci_b200_t *h, int mode) {
     if (int rc = check_handle(h)) return rc;
     if (mode < 0 || mode > 2) return fail(DCI_B200_ERR_ARG, "pruning mode must be 0 (automatic), 1 (always) or 2 (never)");
     h->pruning = mode;
+    return 0;
+}
+
+int dci_b200_set_pruning_limit(dci_b200_t *h, long long max_bytes) {
+    if (int rc = check_handle(h)) return rc;
+    h->pruning_limit = max_bytes < 0 ? ~(size_t)0 : (size_t)max_bytes;
+    if (h->prune.cap > h->pruning_limit) {
+        DeviceGuard g(h->device);
+        DCI_CUDA(cudaDeviceSynchronize());
+        h->prune.release();
+    }
     return 0;
 }
 
@@ -1636,6 +1661,7 @@ int query_noalloc_impl(dci_b200 *h, dci::TraverseParams prm, int nthreads, unsig
     // per query of a pass: its per-partition result lists and its word of the shared distance bound
     const size_t per_query = sizeof(uint64_t) * (size_t)prm.num_parts * prm.kpart + sizeof(uint32_t);
     int prune_first = prune_first_round(h, prm, num_queries);
+    h->last_path = 0;
     if (slabs + per_query + 256 > avail)
         return fail(DCI_B200_ERR_UNSUPPORTED,
                     "this index and k need %zu bytes of working memory, the built-in scratch of the allocation-free query holds %u",

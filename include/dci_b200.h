@@ -221,7 +221,9 @@ int dci_b200_set_max_ctas(dci_b200_t *h, int max_ctas);
 
 /* Which way the handle's last call went, into 8 words; a diagnostic, for tests.
  * [0] kernel of the last projection: 0 rows staged by the computing threads,
- * 1 fed by TMA, 2 the one for few points.  The rest is 0. */
+ * 1 fed by TMA, 2 the one for few points.  [1] the last query: 0 every (query,
+ * partition) pair traversed, 1 only those that distance bounds leave, 2 every row
+ * compared, 3 the groups of rows that bounds leave.  The rest is 0. */
 int dci_b200_last_call(dci_b200_t *h, long long *h_out);
 
 /* Whether queries leave out what provably cannot change their answer: partitions beyond the candidates already
@@ -229,6 +231,13 @@ int dci_b200_last_call(dci_b200_t *h, long long *h_out);
  * (csrc/exhaustive.cuh).  0, the default, where the sizes of the call make it pay; 1 wherever it is possible;
  * 2 never.  Results are the same, bit for bit.  A diagnostic, for tests and comparisons. */
 int dci_b200_set_pruning(dci_b200_t *h, int mode);
+
+/* Device memory that the handle may hold for leaving work out (8 bytes per (query,
+ * partition) pair of a call, at most 1 GiB; 256 MiB where every point is a
+ * candidate).  A call that would need more, or whose allocation fails, traverses
+ * every pair instead.  Negative, the default: no limit.  What is held beyond a new
+ * limit is given back. */
+int dci_b200_set_pruning_limit(dci_b200_t *h, long long max_bytes);
 
 /* How data and queries are projected on the directions (replaces the
  * cublasSgemm calls of src/util_kernel.cu:45-80).  0 (default): exact fp32, one

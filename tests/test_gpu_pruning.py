@@ -121,3 +121,21 @@ def test_answers_do_not_depend_on_what_is_left_out_for_unusual_rows(kind, mc):
             assert torch.equal(out[0][0], o[0]) and torch.equal(out[0][1], o[1])
         return
     _check(data, query, 2, 4, 6, 10, 10, mc, proj, shift=1 if kind == "unaligned" else 0)
+
+
+@pytest.mark.parametrize("mc,path", [(60, "pruned"), (3000, "groups")])
+def test_a_call_goes_without_the_working_memory_it_cannot_have(mc, path):
+    from dciknn_cuda_b200 import DCI
+    rng = np.random.default_rng(9)
+    n, dim, nq, k = 6000, 32, 40, 2
+    z = _rows(rng, n + nq, dim, "latent")
+    g = DCI(dim, 2, 4, 6, 10, proj=torch.from_numpy(cases.unit_rows(rng, 8, dim)))
+    g.add(torch.from_numpy(z[:n]).cuda())
+    q = torch.from_numpy(z[n:]).cuda()
+    out = []
+    for limit, want in ((0, "all"), (None, path), (100, "all"), (1 << 20, path)):
+        g.set_pruning(1, max_bytes=limit)
+        out.append(g.query(q, k, 5000, max_num_candidates=mc, return_int_ids=True))
+        assert g.last_call()["path"] == want, limit
+    for ids, dists in out[1:]:
+        assert torch.equal(ids, out[0][0]) and torch.equal(dists.view(torch.int32), out[0][1].view(torch.int32))
