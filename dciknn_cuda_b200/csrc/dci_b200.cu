@@ -435,22 +435,40 @@ int launch_traverse(dci_b200 *h, dci::TraverseParams prm, int nthreads, cudaStre
     return 0;
 }
 
+// Whether the bounds kernel can read the rows and the queries by TMA (make_tensor_map_2d).
+bool bounds_by_tma(const dci::TraverseParams &prm) {
+    return prm.dim % 4 == 0 && ((uintptr_t)prm.data & 15) == 0 && ((uintptr_t)prm.query & 15) == 0;
+}
+
+// us that the bounds of a call take (launch_bounds).  By TMA: every row read once (6 TB/s), all queries multiplied with
+// all rows (tf32, queries padded to tiles of 128).  Staged by ordinary loads, which every tile of queries does again:
+// 155 455 x 958, 72 queries 675 us; 104 141 x 958, 408 queries 0.88 ms; 78 789 x 958, 1 499 queries 2.5 ms, that is 2.2e5
+// to 4.5e5 coordinates (padded to 32) a us and tile; charged at the latter, since prune_first_round doubles it.
+double bounds_us(const dci::TraverseParams &prm, int num_queries) {
+    const double tiles = (num_queries + dci::kLbQueries - 1) / dci::kLbQueries, cells = (double)prm.N * prm.dim;
+    if (!bounds_by_tma(prm)) return (double)prm.N * ((prm.dim + dci::kLbK - 1) / dci::kLbK * dci::kLbK) * tiles / 4.5e5;
+    return std::max(cells * 4.0 / 6.0e6, cells * tiles * dci::kLbQueries * 2.0 / 0.35e9);
+}
+
 // How a query call decides which (query, partition) pairs to traverse: 0 = all of them, otherwise the number of
 // partitions per query that round 1 visits (prune.cuh).
-// The bounds read every row once (6 TB/s) and multiply all queries with all rows (tf32, queries padded to tiles of
-// 128); a pair that need not be traversed saves about 0.31 ns of one SM per point and simple index (62 us for
-// 10 000 points x 20 indices), and k nearest rows spread evenly over P partitions leave
-// P * (1 - exp(-k / P)) of them to visit.  The factor 2 covers the small launches in between and the last
-// waves of the rounds.
+// A pair that need not be traversed saves about 0.31 ns of one SM per point and simple index (62 us for 10 000 points x
+// 20 indices), and k nearest rows spread evenly over P partitions leave P * (1 - exp(-k / P)) of them to visit.  Where
+// rows are read coordinate by coordinate, the candidates' distances count as well (0.22 ns a coordinate, 0.08 with
+// 256-bit loads; pairs of 2 600 points x 958 take 400 us, 24 of them for the index).  The factor 2 covers the small
+// launches in between, the last waves of the rounds and rows among which nothing can be left out.
+// 154 calls with rows that no tensor map describes, drawn over 10 000 to 2M rows and 1 to 1 500 queries: 0.58 of the time
+// of traversing every pair in the geometric mean, 1.24 at worst (0.62 and 1.58 with the bounds charged as if by TMA;
+// 0.57 if the better way were always known).  166 with rows that TMA reads: 1.14 at worst, uniform rows of unit length.
 int prune_first_round(const dci_b200 *h, const dci::TraverseParams &prm, int num_queries) {
     if (prm.blind || prm.work_stats || prm.phase_cycles || !h->distance_bound || h->pruning == 2) return 0;
     if (prm.num_parts < 2 || prm.ppb < 64) return 0;
     const double parts = prm.num_parts, visited = 1.0 - exp(-1.1 * prm.knn / parts);
-    const double pairs = (double)num_queries * parts;
-    const double saved_us = (1.0 - visited) * pairs * 3.1e-4 * prm.ppb * prm.L * prm.S / h->sm_count;
-    const double padded = (double)((num_queries + dci::kLbQueries - 1) / dci::kLbQueries) * dci::kLbQueries;
-    const double cells = (double)prm.N * prm.dim;
-    const double cost_us = std::max(cells * 4.0 / 6.0e6, cells * padded * 2.0 / 0.35e9) + 40.0;
+    double pair_us = 3.1e-4 * prm.ppb * prm.L * prm.S;
+    if (!bounds_by_tma(prm))
+        pair_us = 2.9 + 3.2e-4 * prm.ppb * prm.L * prm.S +
+                  (prm.vec8 ? 0.8e-4 : 2.2e-4) * std::min<double>(prm.ppb, (double)prm.T * prm.max_cand) * prm.dim;
+    const double saved_us = (1.0 - visited) * num_queries * parts * pair_us / h->sm_count, cost_us = bounds_us(prm, num_queries) + 40.0;
     if (saved_us < 2.0 * cost_us && h->pruning != 1) return 0;
     return std::min(prm.num_parts - 1, std::max(1, (int)(parts * visited + 0.5)));
 }
@@ -640,8 +658,7 @@ ExactPlan plan_exact(const dci_b200 *h, const dci::TraverseParams &prm, int num_
     if (h->pruning == 1) return g;
     if (g.num_groups < 4 * g.first) return p;
     const double scan_us = 8.0 + cells * num_queries * 4.0 / 5.0e6;
-    const double padded = (double)((num_queries + dci::kLbQueries - 1) / dci::kLbQueries) * dci::kLbQueries;
-    const double groups_us = 28.0 + std::max(cells * 4.0 / 6.0e6, cells * padded * 2.0 / 0.35e9) +
+    const double groups_us = 28.0 + bounds_us(prm, num_queries) +
                              2.0 * g.first * g.group_rows * prm.dim * 4.0 / 4.0e4 * std::max(1.0, (double)num_queries / h->sm_count);
     return scan_us > groups_us ? g : p;
 }

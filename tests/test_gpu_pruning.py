@@ -139,3 +139,20 @@ def test_a_call_goes_without_the_working_memory_it_cannot_have(mc, path):
         assert g.last_call()["path"] == want, limit
     for ids, dists in out[1:]:
         assert torch.equal(ids, out[0][0]) and torch.equal(dists.view(torch.int32), out[0][1].view(torch.int32))
+
+
+# 7 queries, k = 1: of rows that no tensor map describes the bounds cost more than the pairs that they leave out; where
+# there are many queries the pairs cost far more
+@pytest.mark.parametrize("n,dim,nq,k,L,S,path", [(501_175, 97, 7, 1, 2, 15, "all"), (501_175, 96, 7, 1, 2, 15, "pruned"),
+                                                 (13_044, 97, 1382, 10, 3, 12, "pruned")])
+def test_bounds_by_ordinary_loads_are_charged_as_such(n, dim, nq, k, L, S, path):
+    from dciknn_cuda_b200 import DCI
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    g = DCI(dim, L, S, 100, 10, seed=1)
+    g.add(torch.randn(n, dim, generator=gen, device="cuda"))
+    q = torch.randn(nq, dim, generator=gen, device="cuda")
+    ids, dists = g.query(q, k, return_int_ids=True)
+    assert g.last_call()["path"] == path
+    g.set_pruning(2)
+    for a, b in zip((ids, dists), g.query(q, k, return_int_ids=True)):
+        assert torch.equal(a.view(torch.int32), b.view(torch.int32))
