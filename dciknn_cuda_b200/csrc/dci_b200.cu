@@ -610,6 +610,10 @@ bool always_exhaustive(const dci::TraverseParams &prm) {
     return true;
 }
 
+// Entries of an exhaustive call's selection buffer: a compaction keeps k of them, and beside one offer of every thread at
+// least 128 more should fit (100 000 x 128, k = 500, 64 queries: 1.6 ms with 1 024 entries, k = 1 000 with 2 048: 0.95).
+int exact_capacity(int knn, int threads) { return std::max(next_pow2(knn + threads), std::min(next_pow2(knn + threads + 128), 2048)); }
+
 // How an exhaustive call is answered (exhaustive.cuh).
 struct ExactPlan {
     int mode = 0;                 // 0: by the traversal, 1: exact_scan_kernel, 2: nearest_groups_kernel
@@ -619,24 +623,37 @@ struct ExactPlan {
     size_t smem = 0, bytes = 0;   // dynamic shared memory; working memory (mode 1: lists, mode 2: bounds and a flag)
 };
 
-// Sizes alone decide.  The scan reads every row once per query (5 TB/s out of L2); the groups read all rows once,
-// multiply them with the padded queries (as in prune_first_round), take two launches more, and one CTA per query then
-// works out about twice `first` groups (40 GB/s each).  Measured with 128 coordinates and k = 10 (us a call): 10 000
-// rows, 8 queries: scan 34, groups 40; 100 queries: 103 and 40; 256 coordinates, k = 100, 100 000 rows, 2 queries: 114
-// and 209; 1 000 queries: 4 663 and 1 214.
+// Sizes alone decide between the scan and the groups.  us of each, as fitted to 870 calls (2 000 to 400 000 rows of 16 to
+// 960 coordinates, 1 to 1 000 queries, k = 10 to 1 000); the second figure of a rate is for rows without 256-bit loads:
+//   scan    rows at 5 TB/s (2.9) or, with few CTAs, 36 GB/s (20) a CTA, 22 (11) where SMs hold two; 0.15 us a neighbour for the
+//           selection; the merge of the slices' lists
+//   groups  the bounds of all rows and two launches more; then a CTA a query: 4 ns a bound, 0.17 us a neighbour and the rows
+//           of k + 8 groups at 35 GB/s (15)
+// Near the lines, 128 coordinates: 100 000 rows, k = 10, 4 queries scan 46, groups 46 us, 16 queries 92 and 52; k = 200, 4
+// queries 148 and 142, 64 queries 708 and 154; k = 1 000, 16 queries 472 and 536, 64 queries 950 and 542.
 ExactPlan plan_exact(const dci_b200 *h, const dci::TraverseParams &prm, int num_queries, size_t avail) {
     ExactPlan p;
     if (prm.blind || prm.work_stats || prm.phase_cycles || h->pruning == 2 || prm.knn > dci::kMaxTopK || prm.dim > 4096 ||
         !always_exhaustive(prm))
         return p;
-    const double cells = (double)prm.N * prm.dim;
+    const double row_bytes = 4.0 * prm.dim, queries_per_sm = (double)num_queries / h->sm_count;
     p.mode = 1;
     p.batch = num_queries;
     p.threads = dci::kScanThreads;
-    p.topk_cap = next_pow2(prm.knn + p.threads);
+    p.topk_cap = exact_capacity(prm.knn, p.threads);
     p.smem = (size_t)p.topk_cap * 16 + (size_t)prm.dim * 4;
-    // slices of at least one row per thread, until every SM has a CTA
-    p.slices = std::max(1, std::min((h->sm_count + num_queries - 1) / num_queries, prm.N / p.threads));
+    // Slices of at least one row per thread, as long as no SM gets a second CTA (20 000 x 128, k = 10, 8 queries: 42 us in
+    // 152 CTAs, 29 in 144), but no more than shortens a slice by as much as it lengthens the merge: a row takes 10 ns and
+    // its bytes, the merge 2 ns an entry and, where the lists are narrowed more than once (merge_capacity), 54 ns a
+    // neighbour (k = 1 000, one query: 2 000 x 16 in 3 slices 60 us, in one 23; 20 000 x 16 in 39 and 10: 179 and 149;
+    // 2 000 x 960 in 3 and one: 122 and 193; k = 300, 2 000 x 50 in 3 and one: 36 and 44).
+    const double row_us = row_bytes / 4.0e4 + 0.01, entry_us = 0.002 * prm.knn;
+    auto merge_us = [&](int slices) {
+        return slices == 1 ? 0.0 : 6.0 + entry_us * slices + (slices * prm.knn + 256 > 2048 ? 0.054 * prm.knn : 0.0);
+    };
+    p.slices = std::max(1, std::min(h->sm_count / num_queries, prm.N / p.threads));
+    p.slices = std::max(1, std::min(p.slices, (int)sqrt(prm.N * row_us / entry_us)));
+    if (prm.N * row_us / p.slices + merge_us(p.slices) > prm.N * row_us) p.slices = 1;
     p.slice_rows = (prm.N + p.slices - 1) / p.slices;
     p.slices = (prm.N + p.slice_rows - 1) / p.slice_rows;
     p.bytes = p.slices > 1 ? sizeof(uint64_t) * (size_t)num_queries * p.slices * prm.knn : 0;
@@ -645,7 +662,7 @@ ExactPlan plan_exact(const dci_b200 *h, const dci::TraverseParams &prm, int num_
     ExactPlan g = p;
     g.mode = 2;
     g.threads = dci::kNgThreads;
-    g.topk_cap = next_pow2(prm.knn + dci::kNgThreads);
+    g.topk_cap = exact_capacity(prm.knn, dci::kNgThreads);
     g.smem = (size_t)g.topk_cap * 16 + (size_t)prm.dim * 4;
     g.group_rows = 32;                                       // the bounds' epilogue takes minima of 32 rows at a time
     while (prm.N / g.group_rows > 32768) g.group_rows *= 2;
@@ -654,12 +671,21 @@ ExactPlan plan_exact(const dci_b200 *h, const dci::TraverseParams &prm, int num_
     const size_t per_query = sizeof(uint32_t) * (size_t)g.num_groups;
     g.batch = (int)std::min<size_t>((size_t)num_queries, (std::min<size_t>(avail, (size_t)256 << 20) - 512) / per_query);
     g.bytes = per_query * g.batch + 512;
-    if (g.num_groups < 2 * g.first || g.batch < 1 || g.bytes > avail || (g.batch < num_queries && g.batch < 1024)) return p;
-    if (h->pruning == 1) return g;
-    if (g.num_groups < 4 * g.first) return p;
-    const double scan_us = 8.0 + cells * num_queries * 4.0 / 5.0e6;
-    const double groups_us = 28.0 + bounds_us(prm, num_queries) +
-                             2.0 * g.first * g.group_rows * prm.dim * 4.0 / 4.0e4 * std::max(1.0, (double)num_queries / h->sm_count);
+    const bool grouped = g.num_groups >= 2 * g.first && g.batch >= 1 && g.bytes <= avail;
+    if (grouped && h->pruning == 1) return g;
+    const bool one_each = (long long)num_queries * p.slices <= h->sm_count;
+    const double scan_us = 8.0 +
+                           std::max((double)prm.N * row_bytes * num_queries / (prm.vec8 ? 5.0e6 : 2.9e6),
+                                    p.slice_rows * row_bytes / (one_each ? (prm.vec8 ? 3.6e4 : 2.0e4) : (prm.vec8 ? 2.2e4 : 1.1e4))) +
+                           0.15 * prm.knn * std::min(1.0, p.slice_rows / (8.0 * prm.knn)) +
+                           merge_us(p.slices);
+    double groups_us = 1.0e30;
+    if (grouped) {
+        const int batches = (num_queries + g.batch - 1) / g.batch;
+        groups_us = batches * (20.0 + bounds_us(prm, std::min(num_queries, g.batch))) +
+                    std::max(queries_per_sm, (double)batches) *
+                        (0.004 * g.num_groups + 0.17 * prm.knn + (prm.knn + 8.0) * g.group_rows * row_bytes / (prm.vec8 ? 3.5e4 : 1.5e4));
+    }
     return scan_us > groups_us ? g : p;
 }
 

@@ -156,3 +156,31 @@ def test_bounds_by_ordinary_loads_are_charged_as_such(n, dim, nq, k, L, S, path)
     g.set_pruning(2)
     for a, b in zip((ids, dists), g.query(q, k, return_int_ids=True)):
         assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+
+
+# exhaustive calls with long lists: one slice or several, both capacities of the selection buffer, as many queries as SMs
+@pytest.mark.parametrize("size", [(2000, 100, 3, 100, 2, 7, 10, 1000, 10_000, "latent"), (2049, 16, 149, 20, 1, 3, 10, 513, 10_000, "mixture"),
+                                  (20_011, 12, 2, 50, 1, 2, 10, 1000, 10_000, "latent"), (1025, 40, 148, 5, 1, 3, 10, 512, 10_000, "unit"),
+                                  (511, 9, 5, 3, 1, 3, 10, 256, 10_000, "unit"), (40_000, 8, 5, 100, 1, 2, 10, 300, 3000, "mixture"),
+                                  (70_001, 16, 20, 100, 1, 2, 10, 257, 3000, "mixture")], ids=lambda s: "%dx%d_q%d" % s[:3])
+def test_exhaustive_calls_with_long_lists(size):
+    n, dim, nq, P, L, S, T, k, mc, dist = size
+    rng = np.random.default_rng(n + k)
+    z = _rows(rng, n + nq, dim, dist)
+    _check(np.ascontiguousarray(z[:n]), np.ascontiguousarray(z[n:]), L, S, P, T, k, mc, cases.unit_rows(rng, L * S, dim))
+
+
+def test_exhaustive_allocation_free_call_in_two_batches():
+    """300 queries against 1M rows: the bounds of all groups do not fit the built-in array at a time, and a scan of every
+    row for every query would take many times as long as two batches of groups."""
+    from dciknn_cuda_b200 import DCI
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    data, q = torch.randn(1_000_000, 8, generator=gen, device="cuda"), torch.randn(300, 8, generator=gen, device="cuda")
+    g = DCI(8, 1, 2, 100, 10, seed=3)
+    g.add(data)
+    ids, dists = torch.empty(300, 10, dtype=torch.int32, device="cuda"), torch.empty(300, 10, device="cuda")
+    g.query_noalloc(q, ids, dists, 5000, max_num_candidates=20_000)
+    assert g.last_call()["path"] == "groups"
+    g.set_pruning(2)
+    for a, b in zip((ids, dists), g.query(q, 10, 5000, max_num_candidates=20_000, return_int_ids=True)):
+        assert torch.equal(a.view(torch.int32), b.view(torch.int32))
