@@ -401,7 +401,8 @@ class DCI(object):
 
     def set_pruning(self, mode, max_bytes=None):
         """0 (default): leave out work that provably cannot change an answer where the sizes of the call make
-        it pay; 1: wherever possible; 2: never.  Results do not depend on it.  max_bytes: device memory that the
+        it pay; 1: wherever possible; 2: never; 3: as 1, but as if a wait of the bounds kernel had run out, which leaves
+        everything in.  Results do not depend on it.  max_bytes: device memory that the
         index may hold for it (None: no limit); a call that needs more goes without."""
         _capi.check(_capi.lib().dci_b200_set_pruning(self._live(), int(mode)))
         _capi.check(_capi.lib().dci_b200_set_pruning_limit(self._live(), -1 if max_bytes is None else int(max_bytes)))
@@ -409,14 +410,28 @@ class DCI(object):
     def last_call(self):
         """Which way the last call went (a diagnostic): the kernel of the last projection, 'staged' (rows staged by
         the computing threads), 'tma' or 'small' (few points), and the path of the last query: 'all' (query, partition)
-        pairs, 'pruned', or, where every point is a candidate, 'scan' (every row) or 'groups' (of rows, by bounds)."""
+        pairs, 'pruned', or, where every point is a candidate, 'scan' (every row) or 'groups' (of rows, by bounds); where
+        work was left out, the batches of the query, and of the last one the rounds, the pairs traversed and whether a
+        wait of the bounds kernel ran out (nothing was left out then)."""
         buf = (C.c_longlong * 8)()
         _capi.check(_capi.lib().dci_b200_last_call(self._live(), buf))
-        return dict(projection=("staged", "tma", "small")[buf[0]], path=("all", "pruned", "scan", "groups")[buf[1]])
+        return dict(projection=("staged", "tma", "small")[buf[0]], path=("all", "pruned", "scan", "groups")[buf[1]],
+                    batches=int(buf[2]), rounds=int(buf[3]), pairs=int(buf[4]), bounds_failed=bool(buf[5]))
+
+    def distance_bounds(self, query, group_rows):
+        """[groups, num_queries] float64: lower bounds of the squared distances between each query and the rows of each
+        run of group_rows rows, by which queries leave work out (a diagnostic)."""
+        self._check_data(query)
+        groups = -(-self.num_points // int(group_rows))
+        out = torch.empty(groups, query.shape[0], dtype=torch.float64, device=query.device)
+        with torch.cuda.device(self._device):
+            _capi.check(_capi.lib().dci_b200_distance_bounds(self._live(), C.c_void_p(query.data_ptr()), query.shape[0], int(group_rows),
+                                                            C.c_void_p(out.data_ptr()), _stream_ptr(self._device)))
+        return out
 
     def set_max_ctas(self, max_ctas):
-        """Caps the number of CTAs of the traversal kernel (0 = automatic).  For tests: with few CTAs
-        every CTA works through many (query, partition) pairs one after the other."""
+        """Caps the number of CTAs of the traversal and of the distance bounds (0 = automatic).  For tests: with
+        few CTAs every CTA works through many (query, partition) pairs or tiles one after the other."""
         _capi.check(_capi.lib().dci_b200_set_max_ctas(self._live(), int(max_ctas)))
 
     def enable_timing(self, on=True):

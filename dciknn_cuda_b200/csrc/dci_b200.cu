@@ -13,6 +13,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <vector>
 #include <atomic>
 #include <mutex>
 #include <new>
@@ -77,6 +78,8 @@ struct DeviceGuard {
     ~DeviceGuard() { if (prev >= 0) cudaSetDevice(prev); }
 };
 
+size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
+
 int next_pow2(int x) { int p = 1; while (p < x) p <<= 1; return p; }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link against libcuda).
@@ -125,9 +128,12 @@ struct dci_b200 {
     Buf keys, ids, pos, keysT;           // sorted index, inverse positions, stride-T keys: L*S*N entries each, partition-major (segment_start)
     int max_ctas = 0;                    // > 0: cap on the traversal grid (dci_b200_set_max_ctas)
     Buf tmp_keys, qproj, part_topk, scratch, merge_scratch, stats, phases, hq, hids, hdists, qbound, prune;
-    int pruning = 0;                     // 0: by the rule of prune_first_round, 1: wherever possible, 2: never
+    int pruning = 0;                     // 0: by the rule of prune_first_round, 1: wherever possible, 2: never, 3: as 1, bounds reported as failed
     size_t pruning_limit = ~(size_t)0;   // bytes that `prune` may take (dci_b200_set_pruning_limit)
     int last_path = 0;                   // of the last query: 0 every pair traversed, 1 pruned, 2 every row, 3 nearest groups
+    int last_rounds = 0, last_batches = 0;       // ... rounds of a pruned query; batches it was taken in
+    const int *last_counts = nullptr, *last_failed = nullptr;     // ... in device memory: pairs listed per round and partition, failure flag
+    int last_num_counts = 0;
     int distance_bound = 1;              // 1: share a per-query distance bound between partitions
     int stats_on = 0, stats_nq = 0, phases_valid = 0;
     int timing_on = 0;
@@ -435,6 +441,8 @@ int launch_traverse(dci_b200 *h, dci::TraverseParams prm, int nthreads, cudaStre
     return 0;
 }
 
+bool always_prune(const dci_b200 *h) { return h->pruning == 1 || h->pruning == 3; }
+
 // Whether the bounds kernel can read the rows and the queries by TMA (make_tensor_map_2d).
 bool bounds_by_tma(const dci::TraverseParams &prm) {
     return prm.dim % 4 == 0 && ((uintptr_t)prm.data & 15) == 0 && ((uintptr_t)prm.query & 15) == 0;
@@ -469,7 +477,7 @@ int prune_first_round(const dci_b200 *h, const dci::TraverseParams &prm, int num
         pair_us = 2.9 + 3.2e-4 * prm.ppb * prm.L * prm.S +
                   (prm.vec8 ? 0.8e-4 : 2.2e-4) * std::min<double>(prm.ppb, (double)prm.T * prm.max_cand) * prm.dim;
     const double saved_us = (1.0 - visited) * num_queries * parts * pair_us / h->sm_count, cost_us = bounds_us(prm, num_queries) + 40.0;
-    if (saved_us < 2.0 * cost_us && h->pruning != 1) return 0;
+    if (saved_us < 2.0 * cost_us && !always_prune(h)) return 0;
     return std::min(prm.num_parts - 1, std::max(1, (int)(parts * visited + 0.5)));
 }
 
@@ -493,6 +501,12 @@ struct PruneSpace {
     }
 };
 
+// A test of what happens when a wait of the bounds kernel runs out: the host sets the flag that the kernel would set.
+int fail_bounds(const dci_b200 *h, int *failed, cudaStream_t st) {
+    if (h->pruning == 3) DCI_CUDA(cudaMemsetAsync(failed, 1, sizeof(int), st));
+    return 0;
+}
+
 // Bounds of every (query, group of rows) of the batch prm.q0 .. prm.q0 + prm.nq.
 int launch_bounds(dci_b200 *h, const dci::TraverseParams &prm, int group_rows, int num_groups, uint32_t *lb, int *failed,
                   cudaStream_t st) {
@@ -511,7 +525,8 @@ int launch_bounds(dci_b200 *h, const dci::TraverseParams &prm, int group_rows, i
     const bool two = q_tiles >= 2 && bp.dim >= 512;
     if (two) bp.qt_per_unit = (bp.qt_per_unit + 1) & ~1;
     bp.units_q = (q_tiles + bp.qt_per_unit - 1) / bp.qt_per_unit;
-    const unsigned grid = (unsigned)std::min<long long>((long long)row_tiles * bp.units_q, h->sm_count);
+    unsigned grid = (unsigned)std::min<long long>((long long)row_tiles * bp.units_q, h->sm_count);
+    if (h->max_ctas > 0) grid = std::min(grid, (unsigned)h->max_ctas);
     CUtensorMap map_x, map_q;
     memset(&map_x, 0, sizeof(map_x));
     memset(&map_q, 0, sizeof(map_q));
@@ -526,6 +541,11 @@ int launch_bounds(dci_b200 *h, const dci::TraverseParams &prm, int group_rows, i
     };
     if (!tma) return go(dci::distance_bounds_kernel<true, 1>, dci::lb_smem(1));
     return two ? go(dci::distance_bounds_kernel<false, 2>, dci::lb_smem(2)) : go(dci::distance_bounds_kernel<false, 1>, dci::lb_smem(1));
+}
+
+void forget_last_query(dci_b200 *h) {
+    h->last_path = h->last_rounds = h->last_batches = h->last_num_counts = 0;
+    h->last_counts = h->last_failed = nullptr;
 }
 
 // Working memory for leaving work out.  A call answers without it just as well, so no memory (or not that much allowed)
@@ -543,6 +563,7 @@ bool pruning_memory(dci_b200 *h, size_t bytes) {
 template <typename Traverse>
 int traverse_pruned(dci_b200 *h, dci::TraverseParams prm, int first, int per_item, long long resident, unsigned char *ws,
                     cudaStream_t st, Traverse traverse) {
+    if (h->max_ctas > 0) resident = std::min<long long>(resident, h->max_ctas);
     // Few pairs: round 1 fills its last wave of CTAs, which costs nothing and leaves less to round 2.  (Rounding down
     // does not pay: with fewer than k partitions the k-th candidate is loose, and round 2 grew by more than the wave.)
     const double waves = (double)prm.nq * first / ((double)resident * per_item);
@@ -553,6 +574,7 @@ int traverse_pruned(dci_b200 *h, dci::TraverseParams prm, int first, int per_ite
     // 1M x 128 go from 71 to 52 ms with two.
     const int rounds = waves < 100.0 ? 2 : (waves < 300.0 ? 3 : 4);
     h->last_path = 1;
+    h->last_batches++;
     const PruneSpace sp = PruneSpace::make(prm.num_parts, prm.nq);
     uint32_t *lb = (uint32_t *)(ws + sp.lb);
     int *zero = (int *)(ws + sp.zero);
@@ -565,6 +587,8 @@ int traverse_pruned(dci_b200 *h, dci::TraverseParams prm, int first, int per_ite
     memset(&s, 0, sizeof(s));
     int *failed = zero + kMaxRounds * prm.num_parts + kMaxRounds;
     if (int rc = launch_bounds(h, prm, prm.ppb, prm.num_parts, lb, failed, st)) return rc;
+    if (int rc = fail_bounds(h, failed, st)) return rc;
+    h->last_rounds = rounds; h->last_counts = zero; h->last_num_counts = kMaxRounds * prm.num_parts; h->last_failed = failed;
     s.lb = lb; s.failed = failed;
     s.query = prm.query + (size_t)prm.q0 * prm.dim;
     s.part_topk = prm.part_topk; s.thresh = (uint32_t *)(ws + sp.thresh); s.qbound = prm.qbound;
@@ -672,7 +696,7 @@ ExactPlan plan_exact(const dci_b200 *h, const dci::TraverseParams &prm, int num_
     g.batch = (int)std::min<size_t>((size_t)num_queries, (std::min<size_t>(avail, (size_t)256 << 20) - 512) / per_query);
     g.bytes = per_query * g.batch + 512;
     const bool grouped = g.num_groups >= 2 * g.first && g.batch >= 1 && g.bytes <= avail;
-    if (grouped && h->pruning == 1) return g;
+    if (grouped && always_prune(h)) return g;
     const bool one_each = (long long)num_queries * p.slices <= h->sm_count;
     const double scan_us = 8.0 +
                            std::max((double)prm.N * row_bytes * num_queries / (prm.vec8 ? 5.0e6 : 2.9e6),
@@ -694,6 +718,7 @@ int launch_exact(dci_b200 *h, const ExactPlan &plan, const dci::TraverseParams &
                  unsigned char *ws, int *d_ids, float *d_dists, unsigned long long *d_packed, cudaStream_t st) {
     h->last_path = plan.mode == 2 ? 3 : 2;
     for (int q0 = 0; q0 < num_queries; q0 += plan.batch) {
+        h->last_batches++;
         dci::ExactParams e;
         memset(&e, 0, sizeof(e));
         e.data = prm.data; e.query = d_query + (size_t)q0 * prm.dim;
@@ -714,6 +739,8 @@ int launch_exact(dci_b200 *h, const ExactPlan &plan, const dci::TraverseParams &
             dci::TraverseParams bp = prm;
             bp.query = d_query; bp.q0 = q0; bp.nq = e.nq;
             if (int rc = launch_bounds(h, bp, plan.group_rows, plan.num_groups, (uint32_t *)ws, failed, st)) return rc;
+            if (int rc = fail_bounds(h, failed, st)) return rc;
+            h->last_failed = failed;
             e.lb = (const uint32_t *)ws; e.failed = failed;
             e.num_groups = plan.num_groups; e.group_rows = plan.group_rows; e.first = plan.first;
             DCI_CUDA(cudaFuncSetAttribute(dci::nearest_groups_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem));
@@ -1062,7 +1089,7 @@ static int query_impl(dci_b200_t *h, const float *d_query, int num_queries, int 
         prm.work_stats = (long long *)h->stats.p;
         h->stats_nq = num_queries;
     }
-    h->last_path = 0;
+    forget_last_query(h);
     const ExactPlan exact = plan_exact(h, prm, num_queries, ~(size_t)0);
     if (exact.mode && pruning_memory(h, exact.bytes)) {      // no index entry is looked at: neither projections nor a traversal
         if (timing) { DCI_CUDA(cudaEventRecord(h->ev[2], st)); }
@@ -1302,6 +1329,20 @@ int dci_b200_last_call(dci_b200_t *h, long long *h_out) {
     for (int i = 0; i < 8; ++i) h_out[i] = 0;
     h_out[0] = h->last_projection;
     h_out[1] = h->last_path;
+    h_out[2] = h->last_batches;
+    h_out[3] = h->last_rounds;
+    DeviceGuard g(h->device);
+    DCI_CUDA(cudaDeviceSynchronize());
+    if (h->last_counts) {
+        std::vector<int> counts(h->last_num_counts);
+        DCI_CUDA(cudaMemcpy(counts.data(), h->last_counts, sizeof(int) * counts.size(), cudaMemcpyDeviceToHost));
+        for (int c : counts) h_out[4] += c;
+    }
+    if (h->last_failed) {
+        int failed = 0;
+        DCI_CUDA(cudaMemcpy(&failed, h->last_failed, sizeof(int), cudaMemcpyDeviceToHost));
+        h_out[5] = failed != 0;
+    }
     return 0;
 }
 
@@ -1318,7 +1359,8 @@ int dci_b200_set_max_ctas(dci_b200_t *h, int max_ctas) {
 
 int dci_b200_set_pruning(dci_b200_t *h, int mode) {
     if (int rc = check_handle(h)) return rc;
-    if (mode < 0 || mode > 2) return fail(DCI_B200_ERR_ARG, "pruning mode must be 0 (automatic), 1 (always) or 2 (never)");
+    if (mode < 0 || mode > 3)
+        return fail(DCI_B200_ERR_ARG, "pruning mode must be 0 (automatic), 1 (always), 2 (never) or 3 (always, bounds reported as failed)");
     h->pruning = mode;
     return 0;
 }
@@ -1330,7 +1372,37 @@ int dci_b200_set_pruning_limit(dci_b200_t *h, long long max_bytes) {
         DeviceGuard g(h->device);
         DCI_CUDA(cudaDeviceSynchronize());
         h->prune.release();
+        forget_last_query(h);
     }
+    return 0;
+}
+
+int dci_b200_distance_bounds(dci_b200_t *h, const float *d_query, int num_queries, int group_rows, double *d_out, void *stream) {
+    if (int rc = check_handle(h)) return rc;
+    if (h->num_points <= 0) return fail(DCI_B200_ERR_STATE, "the index is empty; add data first");
+    if (!d_query || !d_out) return fail(DCI_B200_ERR_ARG, "null query or output pointer");
+    if (num_queries <= 0 || group_rows <= 0) return fail(DCI_B200_ERR_ARG, "num_queries and group_rows must be positive");
+    DeviceGuard g(h->device);
+    cudaStream_t st = (cudaStream_t)stream;
+    const int groups = (int)(((long long)h->num_points + group_rows - 1) / group_rows);
+    const size_t lb_bytes = align256(sizeof(uint32_t) * (size_t)groups * num_queries);
+    DCI_CUDA(h->prune.ensure(lb_bytes + sizeof(int)));
+    forget_last_query(h);
+    uint32_t *lb = (uint32_t *)h->prune.p;
+    int *failed = (int *)((unsigned char *)h->prune.p + lb_bytes);
+    DCI_CUDA(cudaMemsetAsync(lb, 0xFF, lb_bytes, st));
+    DCI_CUDA(cudaMemsetAsync(failed, 0, sizeof(int), st));
+    dci::TraverseParams prm;
+    memset(&prm, 0, sizeof(prm));
+    prm.data = h->d_data; prm.query = d_query; prm.N = h->num_points; prm.dim = h->dim; prm.nq = num_queries;
+    if (int rc = launch_bounds(h, prm, group_rows, groups, lb, failed, st)) return rc;
+    dci::bounds_value_kernel<<<num_queries, 128, 0, st>>>(lb, d_query, h->dim, groups, num_queries, d_out);
+    h->launches++;
+    DCI_CUDA(cudaGetLastError());
+    int flag = 0;
+    DCI_CUDA(cudaMemcpyAsync(&flag, failed, sizeof(int), cudaMemcpyDeviceToHost, st));
+    DCI_CUDA(cudaStreamSynchronize(st));
+    if (flag) return fail(DCI_B200_ERR_CUDA, "distance bounds: a wait on a barrier timed out");
     return 0;
 }
 
@@ -1681,8 +1753,6 @@ int noalloc_scratch_address(int device, unsigned char **out) {
     return 0;
 }
 
-size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
-
 template <typename ValT, typename PosT>
 int query_noalloc_impl(dci_b200 *h, dci::TraverseParams prm, int nthreads, unsigned char *scratch, size_t avail,
                        int num_queries, int *flag_word, int *d_ids, float *d_dists, cudaStream_t st) {
@@ -1704,7 +1774,7 @@ int query_noalloc_impl(dci_b200 *h, dci::TraverseParams prm, int nthreads, unsig
     // per query of a pass: its per-partition result lists and its word of the shared distance bound
     const size_t per_query = sizeof(uint64_t) * (size_t)prm.num_parts * prm.kpart + sizeof(uint32_t);
     int prune_first = prune_first_round(h, prm, num_queries);
-    h->last_path = 0;
+    forget_last_query(h);
     if (slabs + per_query + 256 > avail)
         return fail(DCI_B200_ERR_UNSUPPORTED,
                     "this index and k need %zu bytes of working memory, the built-in scratch of the allocation-free query holds %u",

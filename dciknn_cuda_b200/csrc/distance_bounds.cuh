@@ -1,7 +1,7 @@
 // Lower bounds of the distances between all queries and groups of consecutive rows, on the 5th-generation
 // tensor cores.  A group is a partition of the index (pruning: a partition whose nearest row is provably
 // farther than the k-th candidate found so far cannot change a query's answer, so it is not traversed), or a
-// run of 64 or more rows (exhaustive queries).  No value computed here reaches a result: every returned
+// run of 32 or more rows (exhaustive queries).  No value computed here reaches a result: every returned
 // distance is the fixed fp32 chain of the traversal.
 //
 // For query q and group g the kernel produces

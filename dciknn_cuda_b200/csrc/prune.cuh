@@ -42,6 +42,35 @@ __global__ void prune_init_kernel(uint4 *topk, size_t topk16, uint32_t *lb, size
     for (size_t i = i0; i < (size_t)zero_words; i += step) zero[i] = 0;
 }
 
+// |q|^2 and |dq|^2 (distance_bounds.cuh) of one query, by a CTA of 128 threads; every thread gets both.
+__device__ __forceinline__ void query_norms(const float *__restrict__ q, int dim, double (*sums)[4], double *q2, double *dq2) {
+    double s = 0.0, t = 0.0;
+    for (int c = threadIdx.x; c < dim; c += blockDim.x) {
+        const float v = q[c], e = bounds_residual(v);
+        s += (double)v * v;
+        t += (double)e * e;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) { s += __shfl_xor_sync(0xFFFFFFFFu, s, o); t += __shfl_xor_sync(0xFFFFFFFFu, t, o); }
+    if ((threadIdx.x & 31) == 0) { sums[0][threadIdx.x >> 5] = s; sums[1][threadIdx.x >> 5] = t; }
+    __syncthreads();
+    *q2 = (sums[0][0] + sums[0][1]) + (sums[0][2] + sums[0][3]);
+    *dq2 = (sums[1][0] + sums[1][1]) + (sums[1][2] + sums[1][3]);
+}
+
+// The bounds themselves, for tests: out[g][q] <= |x - q|^2 for every row x of group g; -inf where none is claimed.
+__global__ void __launch_bounds__(128)
+bounds_value_kernel(const uint32_t *__restrict__ lb, const float *__restrict__ query, int dim, int num_groups, int nq, double *__restrict__ out) {
+    __shared__ double s_sum[2][4];
+    const int q = blockIdx.x;
+    double q2, dq2;
+    query_norms(query + (size_t)q * dim, dim, s_sum, &q2, &dq2);
+    for (int g = threadIdx.x; g < num_groups; g += blockDim.x) {
+        const size_t o = (size_t)g * nq + q;
+        out[o] = q2 <= 1.0e30 ? (double)ordered_to_float(lb[o]) + bounds_query_term(q2, dq2, dim) : -(double)__int_as_float(0x7F800000);
+    }
+}
+
 // One CTA per query.  Appends the query to the work lists of the partitions it has to visit in this round; the
 // last CTA to finish turns the list lengths into offsets.
 template <bool FIRST>
@@ -80,18 +109,8 @@ __global__ void __launch_bounds__(128) select_work_kernel(const SelectParams p) 
                 cta_select2([lists](int j) { return (uint32_t)(lists[j] >> 32); }, total, p.knn, p.knn, 32, s_sel, s_res, out);
                 kth = out[0];
             }
-            double s = 0.0, t = 0.0;  // |q|^2 and |dq|^2
-            for (int c = tid; c < p.dim; c += blockDim.x) {
-                const float v = p.query[(size_t)q * p.dim + c], e = bounds_residual(v);
-                s += (double)v * v;
-                t += (double)e * e;
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) { s += __shfl_xor_sync(0xFFFFFFFFu, s, o); t += __shfl_xor_sync(0xFFFFFFFFu, t, o); }
-            if ((tid & 31) == 0) { s_sum[0][tid >> 5] = s; s_sum[1][tid >> 5] = t; }
-            __syncthreads();
-            const double q2 = (s_sum[0][0] + s_sum[0][1]) + (s_sum[0][2] + s_sum[0][3]);
-            const double dq2 = (s_sum[1][0] + s_sum[1][1]) + (s_sum[1][2] + s_sum[1][3]);
+            double q2, dq2;
+            query_norms(p.query + (size_t)q * p.dim, p.dim, s_sum, &q2, &dq2);
             const float d = __uint_as_float(kth);              // an empty slot reads as NaN
             if (d < __int_as_float(0x7F800000) && q2 <= 1.0e30) {
                 // a row is strictly beyond d when its squared distance exceeds d^2 by more than the rounding of

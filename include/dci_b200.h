@@ -214,23 +214,35 @@ long long dci_b200_launch_count(dci_b200_t *h);
  * that a call allocated nothing: the count is the same before and after. */
 long long dci_b200_device_alloc_calls(void);
 
-/* Caps the number of CTAs of the traversal kernel (0, the default: as many as the device keeps
- * resident).  A diagnostic: with few CTAs each one works through many (query, partition) pairs in a
- * row, so tests reach whatever a CTA keeps from one pair to the next. */
+/* Caps the number of CTAs of the traversal kernel and of the distance bounds (0, the default: as many
+ * as the device keeps resident).  A diagnostic: with few CTAs each one works through many (query,
+ * partition) pairs or tiles of rows in a row, so tests reach whatever a CTA keeps from one to the
+ * next, and a pruned query takes more rounds. */
 int dci_b200_set_max_ctas(dci_b200_t *h, int max_ctas);
 
 /* Which way the handle's last call went, into 8 words; a diagnostic, for tests.
  * [0] kernel of the last projection: 0 rows staged by the computing threads,
  * 1 fed by TMA, 2 the one for few points.  [1] the last query: 0 every (query,
  * partition) pair traversed, 1 only those that distance bounds leave, 2 every row
- * compared, 3 the groups of rows that bounds leave.  The rest is 0. */
+ * compared, 3 the groups of rows that bounds leave; [2] the batches it was taken
+ * in where pairs or rows were left out; [3] rounds and [4] pairs traversed of the
+ * last batch of a pruned query; [5] 1 when a wait of its bounds ran out, so that
+ * nothing was left out.  The rest is 0.  Synchronises the device. */
 int dci_b200_last_call(dci_b200_t *h, long long *h_out);
 
 /* Whether queries leave out what provably cannot change their answer: partitions beyond the candidates already
  * known (dciknn_cuda_b200/csrc/prune.cuh), or the whole traversal where every point is a candidate
  * (csrc/exhaustive.cuh).  0, the default, where the sizes of the call make it pay; 1 wherever it is possible;
- * 2 never.  Results are the same, bit for bit.  A diagnostic, for tests and comparisons. */
+ * 2 never; 3 as 1, but as if a wait of the bounds kernel had run out, which leaves
+ * everything in.  Results are the same, bit for bit.  A diagnostic, for tests and
+ * comparisons. */
 int dci_b200_set_pruning(dci_b200_t *h, int mode);
+
+/* The bounds by which work is left out: d_out[g][q], g = 0 .. ceil(n / group_rows) - 1,
+ * is at most the squared distance of query q from any row of the g-th run of
+ * group_rows rows (-inf where none is claimed, +inf for rows without a distance).
+ * A diagnostic, for tests.  Synchronises the stream. */
+int dci_b200_distance_bounds(dci_b200_t *h, const float *d_query, int num_queries, int group_rows, double *d_out, void *stream);
 
 /* Device memory that the handle may hold for leaving work out (8 bytes per (query,
  * partition) pair of a call, at most 1 GiB; 256 MiB where every point is a

@@ -184,3 +184,75 @@ def test_exhaustive_allocation_free_call_in_two_batches():
     g.set_pruning(2)
     for a, b in zip((ids, dists), g.query(q, 10, 5000, max_num_candidates=20_000, return_int_ids=True)):
         assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+
+
+# few CTAs: each of them works through many tiles of the bounds (one and two tiles of queries at a time, ordinary loads)
+# and many listed pairs, and the call takes more rounds
+@pytest.mark.parametrize("max_ctas,rounds", [(1, 4), (3, 3), (40, 2)])
+@pytest.mark.parametrize("size", [(4000, 96, 300, 20, 2, 5, 5, 3, 15, "mixture"), (4001, 50, 280, 20, 3, 5, 7, 3, 30, "mixture"),
+                                  (3000, 516, 300, 10, 1, 3, 10, 2, 20, "mixture")], ids=lambda s: "%dx%d_q%d" % s[:3])
+def test_work_is_left_out_in_every_round(size, max_ctas, rounds):
+    from dciknn_cuda_b200 import DCI
+    n, dim, nq, P, L, S, T, k, mc, dist = size
+    rng = np.random.default_rng(n + dim)
+    z = _rows(rng, n + nq, dim, dist)
+    data, query, proj = np.ascontiguousarray(z[:n]), np.ascontiguousarray(z[n:]), cases.unit_rows(rng, L * S, dim)
+    o = oracle.OracleDCI(dim, L, S, P, T, proj)
+    o.add(data)
+    oi, od = o.query(query, k, 5000, mc)
+    g = DCI(dim, L, S, P, T, proj=torch.from_numpy(proj))
+    g.add(torch.from_numpy(data).cuda())
+    g.set_max_ctas(max_ctas)
+    q = torch.from_numpy(query).cuda()
+    for mode in (1, 3, 2):
+        g.set_pruning(mode)
+        ids, dists = g.query(q, k, 5000, max_num_candidates=mc, return_int_ids=True)
+        last = g.last_call()
+        assert np.array_equal(ids.cpu().numpy(), oi) and np.array_equal(_bits(dists), od.view(np.uint32)), mode
+        if mode == 1:
+            assert last["path"] == "pruned" and last["rounds"] >= rounds and not last["bounds_failed"]
+            assert nq * k // (-(-n // P)) <= last["pairs"] < 0.6 * nq * P, last      # clustered rows: most pairs are left out
+        elif mode == 3:       # the flag of a wait that ran out: everything in the first round
+            assert last["bounds_failed"] and last["pairs"] == nq * P, last
+        else:
+            assert last["path"] == "all"
+
+
+@pytest.mark.parametrize("nq", [1, 129])
+def test_exhaustive_call_with_failed_bounds(nq):
+    from dciknn_cuda_b200 import DCI
+    rng = np.random.default_rng(4)
+    n, dim, k = 6000, 40, 4
+    z = _rows(rng, n + nq, dim, "latent")
+    g = DCI(dim, 1, 3, 4, 10, proj=torch.from_numpy(cases.unit_rows(rng, 3, dim)))
+    g.add(torch.from_numpy(z[:n]).cuda())
+    q = torch.from_numpy(z[n:]).cuda()
+    out = {}
+    for mode in (1, 2, 3):
+        g.set_pruning(mode)
+        out[mode] = g.query(q, k, 5000, max_num_candidates=n, return_int_ids=True)
+        assert (g.last_call()["path"], g.last_call()["bounds_failed"]) == {1: ("groups", False), 2: ("all", False), 3: ("groups", True)}[mode]
+        assert torch.equal(out[mode][0], out[1][0]) and torch.equal(out[mode][1].view(torch.int32), out[1][1].view(torch.int32))
+
+
+# n, dim, nq, L, S, k, max_cand, path: more pairs than the lists of one batch hold (1 GiB), more bounds than fit at a time
+@pytest.mark.parametrize("n,dim,nq,L,S,k,mc,path", [(120_000, 8, 1500, 1, 3, 1000, 1100, "pruned"),
+                                                    (1_000_000, 8, 2300, 1, 2, 10, 20_000, "groups")])
+def test_several_batches_on_a_stream_of_its_own(n, dim, nq, L, S, k, mc, path):
+    from dciknn_cuda_b200 import DCI
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    data, q = torch.randn(n, dim, generator=gen, device="cuda"), torch.randn(nq, dim, generator=gen, device="cuda")
+    g = DCI(dim, L, S, 100, 10, seed=3)
+    g.add(data)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    out = []
+    for mode in (1, 2):
+        g.set_pruning(mode)
+        with torch.cuda.stream(side):
+            out.append(g.query(q, k, 5000, max_num_candidates=mc, return_int_ids=True))
+        side.synchronize()
+        if mode == 1:
+            last = g.last_call()
+            assert last["path"] == path and last["batches"] == 2 and not last["bounds_failed"], last
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1].view(torch.int32), out[1][1].view(torch.int32))
