@@ -44,6 +44,7 @@ SYMBOLS = [
     ("dci_b200_set_max_ctas", C.c_int, [_vp, C.c_int]),
     ("dci_b200_last_call", C.c_int, [_vp, C.POINTER(C.c_longlong)]),
     ("dci_b200_set_pruning", C.c_int, [_vp, C.c_int]),
+    ("dci_b200_always_exhaustive", C.c_int, [C.c_int] * 7),
     ("dci_b200_distance_bounds", C.c_int, [_vp, _vp, C.c_int, C.c_int, _vp, _vp]),
     ("dci_b200_set_pruning_limit", C.c_int, [_vp, C.c_longlong]),
     ("dci_b200_set_projection", C.c_int, [_vp, C.c_int]),

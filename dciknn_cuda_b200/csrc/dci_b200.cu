@@ -1377,6 +1377,19 @@ int dci_b200_set_pruning_limit(dci_b200_t *h, long long max_bytes) {
     return 0;
 }
 
+int dci_b200_always_exhaustive(int num_points, int block_size, int thread_size, int num_simp_indices, int num_neighbours,
+                               int num_outer_iterations, int max_num_candidates) {
+    if (num_points <= 0 || block_size <= 0 || thread_size <= 0 || num_simp_indices <= 0) return 0;
+    dci::TraverseParams prm;
+    memset(&prm, 0, sizeof(prm));
+    prm.N = num_points; prm.T = thread_size; prm.knn = num_neighbours; prm.max_cand = max_num_candidates;
+    prm.ppb = (num_points + block_size - 1) / block_size;
+    prm.num_parts = (num_points + prm.ppb - 1) / prm.ppb;
+    prm.outer_s = (long long)num_outer_iterations * num_simp_indices;
+    prm.wcap = num_simp_indices * ((prm.ppb + thread_size - 1) / thread_size + 2);
+    return always_exhaustive(prm) ? 1 : 0;
+}
+
 int dci_b200_distance_bounds(dci_b200_t *h, const float *d_query, int num_queries, int group_rows, double *d_out, void *stream) {
     if (int rc = check_handle(h)) return rc;
     if (h->num_points <= 0) return fail(DCI_B200_ERR_STATE, "the index is empty; add data first");

@@ -238,6 +238,11 @@ int dci_b200_last_call(dci_b200_t *h, long long *h_out);
  * comparisons. */
 int dci_b200_set_pruning(dci_b200_t *h, int mode);
 
+/* 1 when a query of these sizes makes every point a candidate whatever the data, so that it is
+ * answered without the index, else 0.  Needs no device. */
+int dci_b200_always_exhaustive(int num_points, int block_size, int thread_size, int num_simp_indices, int num_neighbours,
+                               int num_outer_iterations, int max_num_candidates);
+
 /* The bounds by which work is left out: d_out[g][q], g = 0 .. ceil(n / group_rows) - 1,
  * is at most the squared distance of query q from any row of the g-th run of
  * group_rows rows (-inf where none is claimed, +inf for rows without a distance).

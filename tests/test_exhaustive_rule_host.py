@@ -1,17 +1,21 @@
-"""The rule by which a call is answered without the index (always_exhaustive in csrc/dci_b200.cu), restated and checked
-against the sequential restatement: wherever sizes satisfy it, the answer is the exact k nearest rows."""
+"""The rule by which a call is answered without the index (always_exhaustive in csrc/dci_b200.cu, asked through the
+library) against the sequential restatement: wherever sizes satisfy it, the answer is the exact k nearest rows."""
 import numpy as np
 
+from dciknn_cuda_b200 import _capi
 from oracle import oracle
 
 
 def rule(n, parts_wanted, S, T, k, outer, max_cand):
-    ppb = -(-n // parts_wanted)
-    num_parts = -(-n // ppb)
-    wcap = S * (-(-ppb // T) + 2)
-    if max_cand < ppb or max_cand <= k or outer * S < wcap:
-        return False
-    return all(m * T >= -(-m // T) + 2 for m in (ppb, n - (num_parts - 1) * ppb))
+    return bool(_capi.lib().dci_b200_always_exhaustive(n, parts_wanted, T, S, k, outer, max_cand))
+
+
+def test_the_rule_lies_where_it_says():
+    assert rule(2000, 100, 7, 10, 10, 5000, 100)
+    assert not rule(2000, 100, 7, 10, 10, 5000, 19)                       # a quota below a partition
+    assert rule(2000, 100, 7, 10, 10, 4, 20) and not rule(2000, 100, 7, 10, 10, 3, 20)      # iterations: 4 windows a simple index
+    assert rule(2000, 100, 7, 10, 19, 5000, 20) and not rule(2000, 100, 7, 10, 20, 5000, 20)
+    assert not rule(1, 1, 1, 1, 1, 10, 10) and rule(3, 1, 1, 2, 1, 10, 10)      # more iterations than windows: 1 against 3, 6 against 4
 
 
 def test_where_the_rule_holds_the_answer_is_the_exact_one():
