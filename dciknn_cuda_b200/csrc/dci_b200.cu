@@ -450,8 +450,8 @@ bool bounds_by_tma(const dci::TraverseParams &prm) {
 
 // us that the bounds of a call take (launch_bounds).  By TMA: every row read once (6 TB/s), all queries multiplied with
 // all rows (tf32, queries padded to tiles of 128).  Staged by ordinary loads, which every tile of queries does again:
-// 155 455 x 958, 72 queries 675 us; 104 141 x 958, 408 queries 0.88 ms; 78 789 x 958, 1 499 queries 2.5 ms, that is 2.2e5
-// to 4.5e5 coordinates (padded to 32) a us and tile; charged at the latter, since prune_first_round doubles it.
+// 155 455 x 958, 72 queries 665 us; 1M x 97, 8 queries 378 us; 100 003 x 50, 777 queries 166 us, that is 2.2e5 to 3.4e5
+// coordinates (padded to 32) a us and tile; charged at 4.5e5, since prune_first_round doubles it.
 double bounds_us(const dci::TraverseParams &prm, int num_queries) {
     const double tiles = (num_queries + dci::kLbQueries - 1) / dci::kLbQueries, cells = (double)prm.N * prm.dim;
     if (!bounds_by_tma(prm)) return (double)prm.N * ((prm.dim + dci::kLbK - 1) / dci::kLbK * dci::kLbK) * tiles / 4.5e5;
@@ -570,8 +570,9 @@ int traverse_pruned(dci_b200 *h, dci::TraverseParams prm, int first, int per_ite
     if (waves < 16.0)
         first = std::max(first, std::min(prm.num_parts - 1, (int)(ceil(waves) * resident * per_item / prm.nq)));
     // Many pairs: further rounds of a quarter of the first each, since every round brings the k-th candidate down.
-    // Each costs a last wave of CTAs: 67 waves of 1.25M x 96 and 29 of 100k x 50 lose 2 % with one round more, 675 waves of
-    // 1M x 128 go from 71 to 52 ms with two.
+    // Each costs a last wave of CTAs.  Time of two rounds over that of four at 30, 60, 160 and 450 waves: 400 000 x 128 mixture
+    // in 400 partitions, k = 10, 0.88, 0.93, 0.98 and 1.00; 1M x 128 mixture in 100 0.98, 0.97, 0.99 and 1.00, latent rows
+    // 1.15, 1.23, 1.26 and 1.28.  The lines lie where the first no longer loses.
     const int rounds = waves < 100.0 ? 2 : (waves < 300.0 ? 3 : 4);
     h->last_path = 1;
     h->last_batches++;
