@@ -534,6 +534,19 @@ def bench_ours(args):
 
     out = None
     if rank == 0:
+        # the timed step itself: pairs that were traversed, and the distance bounds by which the others were left out
+        local_dci.query(query, cfg["k"], cfg["outer"], max_num_candidates=mc)
+        step = local_dci.last_call()
+        timed_step = {"path": step["path"], "rounds": step["rounds"], "pairs_traversed_last_batch": step["pairs"], "batches": step["batches"]}
+        if step["path"] == "pruned":
+            ppb = -(-local_dci.num_points // cfg["P"])
+            a, b, ms = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True), []
+            for _ in range(4):
+                a.record(); local_dci.distance_bounds(query, ppb); b.record()
+                torch.cuda.synchronize()
+                ms.append(a.elapsed_time(b))
+            timed_step["bounds_ms"] = min(ms[1:])
+            timed_step["bounds_tflops"] = 2.0 * local_dci.num_points * cfg["dim"] * nq / min(ms[1:]) / 1e9
         # roofline of the dominant kernel (traversal): algorithmic bytes from the work counters
         local_dci.enable_work_stats(False, phases=True)
         local_dci.query(query, cfg["k"], cfg["outer"], max_num_candidates=mc)
@@ -587,7 +600,7 @@ def bench_ours(args):
                     "launch_ms": tr_ms, "project_ms": statistics.mean(pj), "merge_ms": statistics.mean(mg),
                     "entries_per_query": entries / nq, "candidates_per_query": cands / nq,
                     "phase_cycles_per_work_item": phase_pw,
-                    "queries_per_pass": phases["queries_per_pass"], "second_bound": second}
+                    "queries_per_pass": phases["queries_per_pass"], "second_bound": second, "timed_step": timed_step}
         cpu_port, cpu_brute, parity = (None, None, None)
         if world == 1 and not args.no_cpu_baseline and args.workload == "configs1":
             cpu_port, cpu_brute, parity = cpu_baselines(local_dci, data_h, query_h, cfg, ids, dists)
