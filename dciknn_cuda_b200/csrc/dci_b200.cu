@@ -451,33 +451,40 @@ bool bounds_by_tma(const dci::TraverseParams &prm) {
 // us that the bounds of a call take (launch_bounds).  By TMA: every row read once (6 TB/s), all queries multiplied with
 // all rows (tf32, queries padded to tiles of 128).  Staged by ordinary loads, which every tile of queries does again:
 // 155 455 x 958, 72 queries 665 us; 1M x 97, 8 queries 378 us; 100 003 x 50, 777 queries 166 us, that is 2.2e5 to 3.4e5
-// coordinates (padded to 32) a us and tile; charged at 4.5e5, since prune_first_round doubles it.
-double bounds_us(const dci::TraverseParams &prm, int num_queries) {
+// coordinates (padded to 32) a us and tile; charged at 5e5, since prune_first_round doubles it.
+double bounds_us(const dci::TraverseParams &prm, int num_queries, bool by_tma) {
     const double tiles = (num_queries + dci::kLbQueries - 1) / dci::kLbQueries, cells = (double)prm.N * prm.dim;
-    if (!bounds_by_tma(prm)) return (double)prm.N * ((prm.dim + dci::kLbK - 1) / dci::kLbK * dci::kLbK) * tiles / 4.5e5;
+    if (!by_tma) return (double)prm.N * ((prm.dim + dci::kLbK - 1) / dci::kLbK * dci::kLbK) * tiles / 5.0e5;
     return std::max(cells * 4.0 / 6.0e6, cells * tiles * dci::kLbQueries * 2.0 / 0.35e9);
 }
 
 // How a query call decides which (query, partition) pairs to traverse: 0 = all of them, otherwise the number of
 // partitions per query that round 1 visits (prune.cuh).
 // A pair that need not be traversed saves about 0.31 ns of one SM per point and simple index (62 us for 10 000 points x
-// 20 indices), and k nearest rows spread evenly over P partitions leave P * (1 - exp(-k / P)) of them to visit.  Where
-// rows are read coordinate by coordinate, the candidates' distances count as well (0.22 ns a coordinate, 0.08 with
-// 256-bit loads; pairs of 2 600 points x 958 take 400 us, 24 of them for the index).  The factor 2 covers the small
-// launches in between, the last waves of the rounds and rows among which nothing can be left out.
-// 154 calls with rows that no tensor map describes, drawn over 10 000 to 2M rows and 1 to 1 500 queries: 0.58 of the time
-// of traversing every pair in the geometric mean, 1.24 at worst (0.62 and 1.58 with the bounds charged as if by TMA;
-// 0.57 if the better way were always known).  166 with rows that TMA reads: 1.14 at worst, uniform rows of unit length.
+// 20 indices), and k nearest rows spread evenly over P partitions leave P * (1 - exp(-k / P)) of them to visit.  The
+// factor 2 covers the small launches in between, the last waves of the rounds and rows among which nothing can be left
+// out.  Rows that no tensor map describes have to pass a second time with what their bounds really cost; a pair saves
+// more there, since its candidates' coordinates are read one by one (0.22 ns each, 0.08 with 256-bit loads, and 0.5 more
+// while they come from HBM, that is until a row is a candidate of several queries: 1M x 97, 8 queries, k = 1 0.41 ms,
+// k = 10 1.29).  154 calls with such rows, drawn over 10 000 to 2M rows and 1 to 1 500 queries, and 234 of a grid: 9 more
+// than 5 % slower than traversing every pair (155 455 x 958 uniform rows of unit length, 72 queries, 1.26 -> 1.93 ms, the
+// others up to 1.19), 16 with the first rule alone (501 175 x 97, 7 queries, 191 -> 301 us).  166 drawn calls with rows
+// that TMA reads: 1.14 at worst, uniform rows of unit length.
 int prune_first_round(const dci_b200 *h, const dci::TraverseParams &prm, int num_queries) {
     if (prm.blind || prm.work_stats || prm.phase_cycles || !h->distance_bound || h->pruning == 2) return 0;
     if (prm.num_parts < 2 || prm.ppb < 64) return 0;
     const double parts = prm.num_parts, visited = 1.0 - exp(-1.1 * prm.knn / parts);
-    double pair_us = 3.1e-4 * prm.ppb * prm.L * prm.S;
-    if (!bounds_by_tma(prm))
-        pair_us = 2.9 + 3.2e-4 * prm.ppb * prm.L * prm.S +
-                  (prm.vec8 ? 0.8e-4 : 2.2e-4) * std::min<double>(prm.ppb, (double)prm.T * prm.max_cand) * prm.dim;
-    const double saved_us = (1.0 - visited) * num_queries * parts * pair_us / h->sm_count, cost_us = bounds_us(prm, num_queries) + 40.0;
-    if (saved_us < 2.0 * cost_us && !always_prune(h)) return 0;
+    const double saved_pairs = (1.0 - visited) * num_queries * parts / h->sm_count;       // of one SM
+    if (!always_prune(h)) {
+        if (saved_pairs * 3.1e-4 * prm.ppb * prm.L * prm.S < 2.0 * (bounds_us(prm, num_queries, true) + 40.0)) return 0;
+        if (!bounds_by_tma(prm)) {
+            const double candidates = std::min<double>(prm.ppb, (double)prm.T * prm.max_cand);
+            const double reuse = std::max(1.0, num_queries * candidates / prm.ppb);
+            const double pair_us = 2.9 + 3.2e-4 * prm.ppb * prm.L * prm.S +
+                                   ((prm.vec8 ? 0.8e-4 : 2.2e-4) + 5.0e-4 / reuse) * candidates * prm.dim;
+            if (saved_pairs * pair_us < 2.0 * (bounds_us(prm, num_queries, false) + 40.0)) return 0;
+        }
+    }
     return std::min(prm.num_parts - 1, std::max(1, (int)(parts * visited + 0.5)));
 }
 
@@ -707,7 +714,7 @@ ExactPlan plan_exact(const dci_b200 *h, const dci::TraverseParams &prm, int num_
     double groups_us = 1.0e30;
     if (grouped) {
         const int batches = (num_queries + g.batch - 1) / g.batch;
-        groups_us = batches * (20.0 + bounds_us(prm, std::min(num_queries, g.batch))) +
+        groups_us = batches * (20.0 + bounds_us(prm, std::min(num_queries, g.batch), bounds_by_tma(prm))) +
                     std::max(queries_per_sm, (double)batches) *
                         (0.004 * g.num_groups + 0.17 * prm.knn + (prm.knn + 8.0) * g.group_rows * row_bytes / (prm.vec8 ? 3.5e4 : 1.5e4));
     }
