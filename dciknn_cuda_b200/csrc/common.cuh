@@ -483,11 +483,21 @@ struct CtaTopK {
     __device__ __forceinline__ void compact() {   // all threads; keeps the k smallest, sorted
         int c = *count;
         __syncthreads();
-        // a short list is cheaper to sort outright; a long one is narrowed first (values that fall into one range
-        // of the histogram stop the narrowing, and the sort takes them all)
+        // a short list is cheaper to sort outright; a long one is narrowed first.  Where one range of the histogram
+        // holds most of the values (a query that is a row itself: 0 beside distances within an octave), the k-th value
+        // itself is looked for (15 000 x 32, 8 such queries: merge 22 us when the sort takes them all)
+        bool exact = false;
         while (c > 128 && c > k + (k >> 2)) {
             const uint64_t *src = buf;
-            const uint32_t tau = cta_cover([src](int j) { return (uint32_t)(src[j] >> 32); }, c, k, sel, res);
+            auto get = [src](int j) { return (uint32_t)(src[j] >> 32); };
+            uint32_t tau;
+            if (exact) {
+                uint32_t t2[2];
+                cta_select2(get, c, k, k, 32, sel, res, t2);
+                tau = t2[0];
+            } else {
+                tau = cta_cover(get, c, k, sel, res);
+            }
             if (threadIdx.x == 0) *count = 0;
             __syncthreads();
             for (int j0 = 0; j0 < c; j0 += blockDim.x) {
@@ -501,7 +511,8 @@ struct CtaTopK {
             const int kept = *count;
             uint64_t *t = buf; buf = other; other = t;
             __syncthreads();
-            if (kept == c) break;
+            if (kept == c && exact) break;      // all the same distance
+            exact = kept > (c >> 1);
             c = kept;
         }
         int len = 2;

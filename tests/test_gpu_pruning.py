@@ -256,3 +256,12 @@ def test_several_batches_on_a_stream_of_its_own(n, dim, nq, L, S, k, mc, path):
             last = g.last_call()
             assert last["path"] == path and last["batches"] == 2 and not last["bounds_failed"], last
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1].view(torch.int32), out[1][1].view(torch.int32))
+
+
+@pytest.mark.parametrize("k,mc", [(10, 100), (1, 30), (100, 5000)])
+def test_queries_that_are_rows(k, mc):
+    """A distance of 0 beside distances within an octave: one range of the selection's histogram holds nearly all."""
+    rng = np.random.default_rng(k)
+    data = cases.unit_uniform(rng, 6000, 32)
+    data[3000:3010] = data[0]
+    _check(data, data[:12].copy(), 1, 5, 40, 10, k, mc, cases.unit_rows(rng, 5, 32))
